@@ -110,6 +110,91 @@ __device__ __forceinline__ T warp_sum(T v) {
   return v;
 }
 
+// ---- accumulators of the transmittance scans --------------------------------
+// FloatPair: the unevaluated sum hi + lo of two floats, |lo| <= ulp(hi) / 2:
+// about 48 significant bits.  It carries the products and sums of long rays
+// (VX_FP32_SCAN_MAX_STEPS), whose results are rounded to one float in the
+// end: GB300 issues an FP64 operation at 1/64 of the FP32 rate, a pair
+// product is seven FP32 operations.  Sums after Knuth (TwoSum) and Dekker
+// (FastTwoSum), products through the exact error of a fused multiply-add.
+// The arithmetic is __f*_rn throughout, so nvcc contracts nothing.  An
+// infinite or NaN result keeps lo = 0 and propagates as the plain float would.
+struct FloatPair {
+  float hi, lo;
+};
+
+__device__ __forceinline__ bool is_finite(float v) { return fabsf(v) <= 3.402823466e38f; }
+
+__device__ __forceinline__ FloatPair pair_fast(float a, float b) {  // |a| >= |b| or a == 0
+  const float s = fadd(a, b);
+  return {s, fsub(b, fsub(s, a))};
+}
+__device__ __forceinline__ FloatPair pair_sum(float a, float b) {
+  const float s = fadd(a, b), t = fsub(s, a);
+  if (!is_finite(s)) return {s, 0.f};
+  return {s, fadd(fsub(a, fsub(s, t)), fsub(b, t))};
+}
+__device__ __forceinline__ FloatPair operator*(FloatPair a, FloatPair b) {
+  const float p = fmul(a.hi, b.hi);
+  if (!is_finite(p)) return {p, 0.f};
+  const float e = __fmaf_rn(a.lo, b.hi, __fmaf_rn(a.hi, b.lo, __fmaf_rn(a.hi, b.hi, -p)));
+  return pair_fast(p, e);
+}
+__device__ __forceinline__ FloatPair operator+(FloatPair a, FloatPair b) {
+  const FloatPair s = pair_sum(a.hi, b.hi);
+  if (!is_finite(s.hi)) return s;
+  return pair_fast(s.hi, fadd(s.lo, fadd(a.lo, b.lo)));
+}
+
+template <typename Acc>
+struct AccOps;
+template <>
+struct AccOps<float> {
+  static __device__ __forceinline__ float of(float v) { return v; }
+  static __device__ __forceinline__ float value(float v) { return v; }
+  static __device__ __forceinline__ float one_minus(float a) { return 1.f - a; }
+  static __device__ __forceinline__ bool below_stop(float v) { return v < 1e-3f; }
+  // gw * T - back / (1 - alpha + 1e-10) of the transmittance backward
+  static __device__ __forceinline__ float grad(float gw_t, float back, float alpha) {
+    return gw_t - back / ((1.f - alpha) + 1e-10f);
+  }
+};
+template <>
+struct AccOps<FloatPair> {
+  static __device__ __forceinline__ FloatPair of(float v) { return {v, 0.f}; }
+  static __device__ __forceinline__ float value(FloatPair v) { return v.hi; }
+  static __device__ __forceinline__ FloatPair one_minus(float a) { return pair_sum(1.f, -a); }
+  static __device__ __forceinline__ bool below_stop(FloatPair v) {
+    const float c = 1e-3f, cl = (float)(1e-3 - (double)1e-3f);
+    return v.hi < c || (v.hi == c && v.lo < cl);
+  }
+  // the quotient from one float division and one correction step, the
+  // difference summed exactly up to its last rounding
+  static __device__ __forceinline__ float grad(float gw_t, FloatPair back, float alpha) {
+    const float c = 1e-10f, cl = (float)(1e-10 - (double)1e-10f);
+    FloatPair d = pair_sum(1.f - alpha, c);
+    d.lo = fadd(d.lo, cl);
+    const float q = fdiv(back.hi, d.hi);
+    if (!is_finite(q)) return gw_t - q;
+    const float r = __fmaf_rn(-q, d.lo, fadd(__fmaf_rn(-q, d.hi, back.hi), back.lo));
+    const FloatPair s = pair_sum(gw_t, -q);
+    return fadd(s.hi, fsub(s.lo, __fdividef(r, d.hi)));
+  }
+};
+
+__device__ __forceinline__ float warp_shfl(float v, int lane) { return __shfl_sync(0xffffffffu, v, lane); }
+__device__ __forceinline__ float warp_shfl_up(float v, int o) { return __shfl_up_sync(0xffffffffu, v, o); }
+__device__ __forceinline__ float warp_shfl_down(float v, int o) { return __shfl_down_sync(0xffffffffu, v, o); }
+__device__ __forceinline__ FloatPair warp_shfl(FloatPair v, int lane) {
+  return {warp_shfl(v.hi, lane), warp_shfl(v.lo, lane)};
+}
+__device__ __forceinline__ FloatPair warp_shfl_up(FloatPair v, int o) {
+  return {warp_shfl_up(v.hi, o), warp_shfl_up(v.lo, o)};
+}
+__device__ __forceinline__ FloatPair warp_shfl_down(FloatPair v, int o) {
+  return {warp_shfl_down(v.hi, o), warp_shfl_down(v.lo, o)};
+}
+
 // Inclusive warp prefix product (Hillis-Steele; 5 shuffle rounds).
 template <typename T>
 __device__ __forceinline__ T warp_inclusive_prod(T v) {

@@ -3,88 +3,115 @@
 // Drop-in for render_utils_cuda.alpha2weight / alpha2weight_backward
 // (render_utils.cpp:182-183; kernels render_utils_kernel.cu:577-707).  The
 // reference walks each ray with one thread (8192 rays -> 32 CTAs on 152 SMs)
-// and a serial loop.  Here one warp owns one ray and walks it 32 samples at a
-// time with a warp prefix product; the running transmittance is carried in
-// FP64 on segments of more than 512 samples (so the prefix stays accurate on
-// rays of thousands of samples) and in FP32 on shorter ones, as the
-// reference's float loop.  Semantics kept exactly:
+// and a serial loop.  Here one warp owns one ray and walks it 128 samples at
+// a time: four 32-sample prefix products that do not depend on one another,
+// then the running transmittance through the four.  It is carried as a
+// FloatPair on segments of more than 512 samples (so the prefix stays
+// accurate on rays of thousands of samples) and in FP32 on shorter ones, as
+// the reference's float loop.  Semantics kept exactly:
 //   T[i] = prod_{j<i} (1 - alpha[j]),  w[i] = T[i] * alpha[i],
 //   stop after the first sample whose inclusive product drops below 1e-3,
 //   samples after the stop keep w = 0, T = 1, grad = 0,
 //   empty rays report i_start = i_end = 0 and alphainv_last = 1.
-// Segment bounds come from a binary search in the sorted ray_id instead of
-// the reference's scatter kernel + device-indexed host write (:607-635).
+// Segment bounds come from a search in the sorted ray_id instead of the
+// reference's scatter kernel + device-indexed host write (:607-635).
+//
+// Bound: the latency of a ray's chain (search, loads, scans); the bytes (24
+// a sample forward, 24 backward) would take 14 us at 8192 rays x 400
+// samples.  Forward and backward there, with the host's two calls: 178 us
+// with 32 samples a step, a bisection per bound and FP64 beyond 512 samples
+// (62 + 105 us of kernels), 74 us now, where the calls themselves take as
+// long as the kernels.
 #include "common.cuh"
 
 namespace vx {
 
-// Segment [beg, end) of ray r in a sorted ray_id array.
+// Segment [beg, end) of ray r in a sorted ray_id array.  Each half of the
+// warp searches one bound, sixteen probes a step: six dependent loads for
+// millions of samples, where a bisection takes 22.
 __device__ __forceinline__ void ray_segment(const int64_t* __restrict__ ray_id, int64_t n_pts, int64_t r,
                                             int64_t* beg, int64_t* end) {
-  // Lanes 0 and 1 search the two bounds concurrently.
-  const int lane = lane_id();
-  int64_t v = 0;
-  if (lane < 2) v = lower_bound_i64(ray_id, 0, n_pts, r + lane);
-  *beg = __shfl_sync(0xffffffffu, v, 0);
-  *end = __shfl_sync(0xffffffffu, v, 1);
+  const int lane = lane_id(), half = lane >> 4, sub = lane & 15;
+  const int64_t key = r + half;
+  int64_t lo = 0, hi = n_pts;
+  while (__any_sync(0xffffffffu, lo < hi)) {
+    const int64_t n = hi - lo;
+    // n * (sub + 1) / 17 without the overflow, always below n
+    const int64_t at = lo + n / 17 * (sub + 1) + n % 17 * (sub + 1) / 17;
+    const bool less = lo < hi && ray_id[at] < key;
+    const int c = __popc((__ballot_sync(0xffffffffu, less) >> (16 * half)) & 0xffffu);
+    const int64_t below = __shfl_sync(0xffffffffu, at, 16 * half + max(c - 1, 0));
+    const int64_t above = __shfl_sync(0xffffffffu, at, 16 * half + min(c, 15));
+    if (lo < hi) {
+      if (c > 0) lo = below + 1;
+      if (c < 16) hi = above;
+    }
+  }
+  *beg = __shfl_sync(0xffffffffu, lo, 0);
+  *end = __shfl_sync(0xffffffffu, lo, 16);
 }
 
+constexpr int CHUNKS = 4;   // 32-sample scans in flight per warp
+
 // Warp-level forward scan of one segment.  Writes weight/T for every sample
-// of [beg, end); returns (via lane 0 convention, broadcast) i_end and
-// alphainv_last.
+// of [beg, end); returns i_end and alphainv_last in every lane.
 template <typename Acc>
 __device__ __forceinline__ void scan_segment_fwd(const float* __restrict__ alpha, int64_t beg, int64_t end,
                                                  float* __restrict__ weight, float* __restrict__ T,
                                                  int64_t* i_end_out, float* last_out) {
+  using Op = AccOps<Acc>;
   const int lane = lane_id();
-  Acc carry = 1;
-  bool stopped = false;
-  int64_t i_end = end;
-  float last = 1.f;
-  for (int64_t base = beg; base < end; base += 32) {
-    const int64_t i = base + lane;
-    const bool valid = i < end;
-    if (stopped) {
-      if (valid) {
-        weight[i] = 0.f;
-        T[i] = 1.f;
-      }
-      continue;
+  Acc carry = Op::of(1.f);
+  float nxt[CHUNKS];
+#pragma unroll
+  for (int c = 0; c < CHUNKS; ++c) nxt[c] = beg + 32 * c + lane < end ? alpha[beg + 32 * c + lane] : 0.f;
+  for (int64_t base = beg; base < end; base += 32 * CHUNKS) {
+    float a[CHUNKS];
+    Acc incl[CHUNKS];
+#pragma unroll
+    for (int c = 0; c < CHUNKS; ++c) {
+      a[c] = nxt[c];
+      incl[c] = Op::one_minus(a[c]);
+      const int64_t i = base + 32 * (CHUNKS + c) + lane;   // the next step's samples, while this one scans
+      nxt[c] = i < end ? alpha[i] : 0.f;
     }
-    const float a = valid ? alpha[i] : 0.f;
-    const Acc f = Acc(1) - (Acc)a;
-    const Acc incl = warp_inclusive_prod(f) * carry;
-    Acc excl = __shfl_up_sync(0xffffffffu, incl, 1);
-    if (lane == 0) excl = carry;
-    const unsigned stop_mask = __ballot_sync(0xffffffffu, valid && incl < Acc(1e-3));
-    if (stop_mask) {
-      const int k = __ffs(stop_mask) - 1;  // first sample that drops below 1e-3
-      const Acc incl_k = __shfl_sync(0xffffffffu, incl, k);
-      if (valid) {
-        if (lane <= k) {
-          const float t = (float)excl;
-          T[i] = t;
-          weight[i] = t * a;
-        } else {
-          weight[i] = 0.f;
-          T[i] = 1.f;
-        }
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1)
+#pragma unroll
+      for (int c = 0; c < CHUNKS; ++c) {
+        const Acc u = warp_shfl_up(incl[c], o);
+        if (lane >= o) incl[c] = incl[c] * u;
       }
-      stopped = true;
-      i_end = base + k + 1;
-      last = (float)incl_k;
-    } else {
+#pragma unroll
+    for (int c = 0; c < CHUNKS; ++c) {
+      const int64_t first = base + 32 * c, i = first + lane;
+      if (first >= end) break;
+      const bool valid = i < end;
+      const Acc v = incl[c] * carry;
+      Acc excl = warp_shfl_up(v, 1);
+      if (lane == 0) excl = carry;
+      const unsigned stop_mask = __ballot_sync(0xffffffffu, valid && Op::below_stop(v));
+      // the first sample that drops below 1e-3 is the last one with a weight
+      const int k = stop_mask ? __ffs(stop_mask) - 1 : 31;
       if (valid) {
-        const float t = (float)excl;
+        const float t = lane <= k ? Op::value(excl) : 1.f;
         T[i] = t;
-        weight[i] = t * a;
+        weight[i] = lane <= k ? t * a[c] : 0.f;
       }
-      carry = __shfl_sync(0xffffffffu, incl, 31);
+      carry = warp_shfl(v, k);
+      if (stop_mask) {
+        for (int64_t j = i + 32; j < end; j += 32) {
+          weight[j] = 0.f;
+          T[j] = 1.f;
+        }
+        *i_end_out = first + k + 1;
+        *last_out = Op::value(carry);
+        return;
+      }
     }
   }
-  if (!stopped) last = (float)carry;
-  *i_end_out = i_end;
-  *last_out = last;
+  *i_end_out = end;
+  *last_out = Op::value(carry);
 }
 
 __global__ void alpha2weight_kernel(const float* __restrict__ alpha, const int64_t* __restrict__ ray_id,
@@ -106,7 +133,7 @@ __global__ void alpha2weight_kernel(const float* __restrict__ alpha, const int64
   int64_t ie;
   float last;
   if (end - beg > VX_FP32_SCAN_MAX_STEPS)
-    scan_segment_fwd<double>(alpha, beg, end, weight, T, &ie, &last);
+    scan_segment_fwd<FloatPair>(alpha, beg, end, weight, T, &ie, &last);
   else
     scan_segment_fwd<float>(alpha, beg, end, weight, T, &ie, &last);
   if (lane_id() == 0) {
@@ -119,35 +146,49 @@ __global__ void alpha2weight_kernel(const float* __restrict__ alpha, const int64
 // Reverse scan, render_utils_kernel.cu:671-675:
 //   back = grad_last*alphainv_last;  for i = i_end-1 .. i_start:
 //     grad[i] = gw[i]*T[i] - back/(1-alpha[i]+1e-10);  back += gw[i]*w[i]
-// The running sum `back` is carried in Acc (FP64 on segments of more than
-// 512 samples).
+// The running sum `back` is carried in Acc (a FloatPair on segments of more
+// than 512 samples).
 template <typename Acc>
 __device__ __forceinline__ void scan_segment_bwd(const float* __restrict__ alpha, const float* __restrict__ weight,
                                                  const float* __restrict__ T, const float* __restrict__ grad_w,
                                                  int64_t beg, int64_t end, float back0,
                                                  float* __restrict__ grad) {
+  using Op = AccOps<Acc>;
   const int lane = lane_id();
-  Acc carry = (Acc)back0;
-  for (int64_t top = end; top > beg; top -= 32) {
-    const int64_t i = top - 32 + lane;
-    const bool valid = i >= beg;
-    float gw = 0.f, w = 0.f, t = 0.f, a = 0.f;
-    if (valid) {
-      gw = grad_w[i];
-      w = weight[i];
-      t = T[i];
-      a = alpha[i];
+  Acc carry = Op::of(back0);
+  for (int64_t top = end; top > beg; top -= 32 * CHUNKS) {
+    float gw_t[CHUNKS], a[CHUNKS];
+    Acc suffix[CHUNKS];
+#pragma unroll
+    for (int c = 0; c < CHUNKS; ++c) {
+      const int64_t i = top - 32 * (c + 1) + lane;
+      float gw = 0.f, w = 0.f, t = 0.f;
+      a[c] = 0.f;
+      if (i >= beg) {
+        gw = grad_w[i];
+        w = weight[i];
+        t = T[i];
+        a[c] = alpha[i];
+      }
+      gw_t[c] = gw * t;
+      suffix[c] = Op::of(i >= beg ? gw * w : 0.f);
     }
-    const Acc term = valid ? (Acc)(gw * w) : Acc(0);
-    const Acc suffix = warp_inclusive_suffix_sum(term);  // sum of lanes >= this lane
-    Acc after = __shfl_down_sync(0xffffffffu, suffix, 1);
-    if (lane == 31) after = 0;
-    const Acc back = carry + after;
-    if (valid) {
-      const Acc denom = (Acc)(1.f - a) + Acc(1e-10);
-      grad[i] = (float)((Acc)(gw * t) - back / denom);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1)
+#pragma unroll
+      for (int c = 0; c < CHUNKS; ++c) {
+        const Acc u = warp_shfl_down(suffix[c], o);
+        if (lane + o < 32) suffix[c] = suffix[c] + u;
+      }
+#pragma unroll
+    for (int c = 0; c < CHUNKS; ++c) {
+      const int64_t i = top - 32 * (c + 1) + lane;
+      Acc after = warp_shfl_down(suffix[c], 1);   // the lanes above this one
+      if (lane == 31) after = Op::of(0.f);
+      const Acc back = carry + after;
+      if (i >= beg) grad[i] = Op::grad(gw_t[c], back, a[c]);
+      carry = carry + warp_shfl(suffix[c], 0);
     }
-    carry += __shfl_sync(0xffffffffu, suffix, 0);
   }
 }
 
@@ -168,7 +209,7 @@ __global__ void alpha2weight_backward_kernel(const float* __restrict__ alpha, co
     return;
   }
   if (end - beg > VX_FP32_SCAN_MAX_STEPS)
-    scan_segment_bwd<double>(alpha, weight, T, grad_weights, beg, end, grad_last[r] * alphainv_last[r], grad);
+    scan_segment_bwd<FloatPair>(alpha, weight, T, grad_weights, beg, end, grad_last[r] * alphainv_last[r], grad);
   else
     scan_segment_bwd<float>(alpha, weight, T, grad_weights, beg, end, grad_last[r] * alphainv_last[r], grad);
 }
