@@ -1217,6 +1217,61 @@ __global__ void grid_sample_bwd_kernel(const float* __restrict__ grad_out, int C
   }
 }
 
+// Channel-last grids with C % 4 == 0 (k0): a thread per point and float4 of
+// channels, so that the C / 4 threads of a point read each corner voxel as
+// one run of 4 C bytes and the output rows leave whole.  The scalar kernel
+// above reads 4 bytes of 32 different voxels per instruction.  Same corner
+// order and weights, so the values are the same bits.  Bound: gathers of the
+// corners from L2 and DRAM.  700,003 points, 12 channels, 256^3: 221 -> 46 us.
+__global__ void __launch_bounds__(256) grid_sample_vec_kernel(const float4* __restrict__ grid, int quads, GridGeom g,
+                                                              const float* __restrict__ xyz, int64_t n,
+                                                              float4* __restrict__ out) {
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= n * quads) return;
+  const int64_t i = t / quads;
+  const int v = (int)(t - i * quads);
+  const float p[3] = {xyz[3 * i], xyz[3 * i + 1], xyz[3 * i + 2]};
+  float ind[3];
+  to_index(g, p, ind);
+  const Corners c = corners_of(g, ind[0], ind[1], ind[2]);
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    if (c.off[q] < 0) continue;
+    const float4 x = __ldg(grid + (int64_t)c.off[q] * quads + v);
+    acc.x += c.w[q] * x.x;
+    acc.y += c.w[q] * x.y;
+    acc.z += c.w[q] * x.z;
+    acc.w += c.w[q] * x.w;
+  }
+  out[t] = acc;
+}
+
+// Its adjoint: one 16-byte reduction per corner, point and float4 in place of
+// four scalar ones.  Bound: the rate of L2 reductions; 389 -> 85 us at the
+// sizes above (93 us with a thread per point and the contributions of a
+// warp's points to a voxel summed first).
+__global__ void __launch_bounds__(256) grid_sample_vec_bwd_kernel(const float4* __restrict__ grad_out, int quads,
+                                                                  GridGeom g, const float* __restrict__ xyz,
+                                                                  int64_t n, float* __restrict__ grad_grid) {
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= n * quads) return;
+  const int64_t i = t / quads;
+  const int v = (int)(t - i * quads);
+  const float4 d = grad_out[t];
+  if (d.x == 0.f && d.y == 0.f && d.z == 0.f && d.w == 0.f) return;
+  const float p[3] = {xyz[3 * i], xyz[3 * i + 1], xyz[3 * i + 2]};
+  float ind[3];
+  to_index(g, p, ind);
+  const Corners c = corners_of(g, ind[0], ind[1], ind[2]);
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    if (c.off[q] < 0 || c.w[q] == 0.f) continue;
+    const float w = c.w[q];
+    red_add_v4(grad_grid + 4 * ((int64_t)c.off[q] * quads + v), w * d.x, w * d.y, w * d.z, w * d.w);
+  }
+}
+
 }  // namespace vx
 
 using namespace vx;
@@ -1237,12 +1292,24 @@ static GridGeom geom_from(const vx_grid_geom* gg) {
   return g;
 }
 
+// The float4 kernels take a channel-last grid of whole float4s whose pointers
+// are 16-byte aligned (a torch view may start anywhere).
+static bool vec_layout(int64_t C, int channel_last, const void* a, const void* b) {
+  return channel_last && C % 4 == 0 && ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 15) == 0;
+}
+
 int vx_grid_sample(const float* grid, int64_t C, int channel_last, const vx_grid_geom* geom, const float* xyz,
                    int64_t n_pts, float* out, void* stream) {
   if (!geom || C <= 0 || n_pts < 0) return VX_ERR_ARG;
   if (n_pts == 0) return VX_OK;
   if (!grid || !xyz || !out) return VX_ERR_ARG;
   if (geom->X * geom->Y * geom->Z > INT32_MAX) return VX_ERR_ARG;
+  if (vec_layout(C, channel_last, grid, out)) {
+    grid_sample_vec_kernel<<<grid_for(n_pts * (C / 4), 256), 256, 0, as_stream(stream)>>>(
+        reinterpret_cast<const float4*>(grid), (int)(C / 4), geom_from(geom), xyz, n_pts,
+        reinterpret_cast<float4*>(out));
+    return launch_status();
+  }
   grid_sample_kernel<<<grid_for(n_pts, 128), 128, 0, as_stream(stream)>>>(grid, (int)C, channel_last,
                                                                          geom_from(geom), xyz, n_pts, out);
   return launch_status();
@@ -1254,6 +1321,11 @@ int vx_grid_sample_backward(const float* grad_out, int64_t C, int channel_last, 
   if (n_pts == 0) return VX_OK;
   if (!grad_out || !xyz || !grad_grid) return VX_ERR_ARG;
   if (geom->X * geom->Y * geom->Z > INT32_MAX) return VX_ERR_ARG;
+  if (vec_layout(C, channel_last, grad_out, grad_grid)) {
+    grid_sample_vec_bwd_kernel<<<grid_for(n_pts * (C / 4), 256), 256, 0, as_stream(stream)>>>(
+        reinterpret_cast<const float4*>(grad_out), (int)(C / 4), geom_from(geom), xyz, n_pts, grad_grid);
+    return launch_status();
+  }
   grid_sample_bwd_kernel<<<grid_for(n_pts, 128), 128, 0, as_stream(stream)>>>(grad_out, (int)C, channel_last,
                                                                              geom_from(geom), xyz, n_pts, grad_grid);
   return launch_status();
