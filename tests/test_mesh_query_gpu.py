@@ -70,3 +70,26 @@ def test_extract_geometry_needs_a_host_mesher(cuda):
         return
     v, t = model.extract_geometry(model.xyz_min, model.xyz_max, resolution=20)
     assert len(t) > 0 and np.all(v >= model.xyz_min.cpu().numpy() - 1e-6)
+
+
+@pytest.mark.parametrize("R", [1, 2, 15, 16, 17, 127, 129, 258])
+@pytest.mark.parametrize("shape", [(1, 1, 1), (2, 3, 40), (33, 17, 65)])
+def test_field_tiles_vs_fp64(cuda, shape, R):
+    """Lattices at the edges of the kernel's tiles (4 i x 16 j x 128 k), finer
+    and coarser than the grid, with a box that reaches outside it."""
+    sdf = torch.randn(shape, generator=torch.Generator().manual_seed(R)).to(cuda)
+    bmin, bmax = (-0.5, -1.0, -1.2), (1.0, 1.3, 1.0)
+    u = extract_fields(sdf, torch.tensor([-1.0] * 3), torch.tensor([1.0] * 3), bmin, bmax, R)
+    axes = [torch.linspace(a, b, R).double() for a, b in zip(bmin, bmax)]
+    pts = torch.stack(torch.meshgrid(*axes, indexing="ij"), -1).flip(-1)[None].to(cuda)
+    ref = -torch.nn.functional.grid_sample(sdf.double()[None, None], pts, mode="bilinear", padding_mode="zeros",
+                                           align_corners=True)[0, 0]
+    # an FP32 index in voxels is off by up to about 5 ulp of the grid's size (four
+    # roundings of world_to_index, one of the lattice), each voxel difference up
+    # to 2 max|sdf| per axis; the eight-term sum rounds another 10 times
+    peak = float(sdf.abs().max())
+    bound = (3 * 2 * 5 * max(shape) + 10) * 2.0 ** -24 * peak
+    # on the box's own faces the rounded index decides between the border voxel
+    # and the zero outside
+    edge = ((pts[0].abs() - 1).abs() < 1e-6).any(-1)
+    assert float((u.double() - ref)[~edge].abs().max() if (~edge).any() else 0.0) <= bound

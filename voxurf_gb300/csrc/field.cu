@@ -5,7 +5,7 @@
 // query_func = grid_sampler(pts, -sdf_grid) on the R^3 lattice
 // torch.linspace(bound_min[a], bound_max[a], R) per axis (meshgrid 'ij'),
 // in 64^3 chunks with a host copy per chunk.  Here one launch writes the
-// whole [R, R, R] field on the device: a thread per lattice point, the
+// whole [R, R, R] field on the device: a thread per column of lattice points, the
 // lattice coordinate formed as torch.linspace forms it (start + step * i for
 // the first half, end - step * (R - 1 - i) for the second), then the
 // trilinear lookup (align_corners, zero padding) scaled by `sign`.
@@ -78,56 +78,134 @@ __device__ __forceinline__ float lattice(const FieldAxis& a, int i, int R) {
   return i < a.half ? fadd(a.start, fmul(a.step, (float)i)) : fsub(a.end, fmul(a.step, (float)(R - 1 - i)));
 }
 
-// One warp per lattice row (i, j): the x/y part of the trilinear lookup
-// (floors, weights, the four row offsets and their bounds) is formed once
-// per row, the lanes walk z (consecutive lattice points, coalesced stores).
-// Corner order and weight products are those of corners_of / gather1, so a
-// point's value is bit-identical to sample1 at the same index.
-__global__ void __launch_bounds__(256) sdf_field_kernel(const float* __restrict__ sdf, GridGeom g, FieldAxis ax,
-                                                        FieldAxis ay, FieldAxis az, int R, float sign,
-                                                        float* __restrict__ out) {
-  const int lane = threadIdx.x & 31;
-  const int64_t rows = (int64_t)R * R;
-  const int64_t wstride = (int64_t)gridDim.x * (blockDim.x >> 5);
-  for (int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); row < rows; row += wstride) {
-    const int i = (int)(row / R), j = (int)(row - (int64_t)i * R);
-    const float fi = world_to_index(g, 0, lattice(ax, i, R));
-    const float fj = world_to_index(g, 1, lattice(ay, j, R));
-    const float fi0 = floorf(fi), fj0 = floorf(fj);
-    const int i0 = (int)fi0, j0 = (int)fj0;
-    const float ti = fi - fi0, tj = fj - fj0;
-    const float wi[2] = {1.f - ti, ti}, wj[2] = {1.f - tj, tj};
-    int64_t rbase[2][2];
-    bool rin[2][2];
+// A CTA owns FIELD_NI i, FIELD_ROWS consecutive j and 128 consecutive k of the
+// lattice; a thread walks the rows at its own k for all the CTA's i.  Its x and
+// z corners and their weight products are formed once, the rows' y corners and
+// weights once per CTA (shared memory).  A grid row's four x-z corners are
+// summed when the walk reaches it, and a point is the y-weighted sum of two
+// such rows: where the lattice is twice as fine as the grid that is two loads
+// and four multiply-adds a point, instead of eight gathers, sixteen
+// multiply-adds and a division.
+// Bound: the 4 bytes written per point and instruction issue.  512^3 points of
+// a 256^3 grid: 771 us with a warp per lattice row and eight gathers a point,
+// 226 us with the corner values kept over the walk but all eight weighted for
+// each point, 164 us now.  (4 i and 16 rows: 8 rows 182 us, 32 rows 168 us, 2 i
+// 170 us; the next grid row loaded ahead 179 us.)
+constexpr int FIELD_NI = 4;
+constexpr int FIELD_ROWS = 16;
+constexpr int FIELD_THREADS = 128;
+
+// A thread's x and z corners: column offsets, weights, and whether the corner
+// (bit 4 p + 2 di + dk) lies in the grid; the others count as zero.
+struct FieldCols {
+  int col[FIELD_NI][2];
+  float wi[FIELD_NI][2], wk[2];
+  unsigned inside;
+};
+
+// ALL: every corner of the CTA's rows is inside.
+template <bool ALL>
+__device__ __forceinline__ void field_load(const float* __restrict__ sdf, const GridGeom& g, int jj,
+                                           const FieldCols& c, float (&v)[FIELD_NI][2][2]) {
+  const bool in_j = jj >= 0 && jj < g.Y;
+  const float* row = sdf + (ALL || in_j ? jj : 0) * g.Z;
+#pragma unroll
+  for (int p = 0; p < FIELD_NI; ++p)
 #pragma unroll
     for (int di = 0; di < 2; ++di)
 #pragma unroll
-      for (int dj = 0; dj < 2; ++dj) {
-        const int ii = i0 + di, jj = j0 + dj;
-        rin[di][dj] = (ii >= 0) & (ii < g.X) & (jj >= 0) & (jj < g.Y);
-        rbase[di][dj] = ((int64_t)ii * g.Y + jj) * g.Z;
+      for (int dk = 0; dk < 2; ++dk)
+        v[p][di][dk] = ALL || (in_j && ((c.inside >> (4 * p + 2 * di + dk)) & 1u)) ? __ldg(row + c.col[p][di] + dk) : 0.f;
+}
+
+__device__ __forceinline__ void field_sum(const FieldCols& c, const float (&v)[FIELD_NI][2][2],
+                                          float (&sum)[FIELD_NI]) {
+#pragma unroll
+  for (int p = 0; p < FIELD_NI; ++p)
+    sum[p] = c.wi[p][0] * (c.wk[0] * v[p][0][0] + c.wk[1] * v[p][0][1]) +
+             c.wi[p][1] * (c.wk[0] * v[p][1][0] + c.wk[1] * v[p][1][1]);
+}
+
+template <bool ALL>
+__device__ __forceinline__ void field_walk(const float* __restrict__ sdf, const GridGeom& g,
+                                           const float2* __restrict__ row_w, const int* __restrict__ row_j0, int rows,
+                                           int n_i, int64_t R, const FieldCols& c, float* __restrict__ o) {
+  float lo[FIELD_NI], hi[FIELD_NI], v[FIELD_NI][2][2];
+  int at = row_j0[0];
+  field_load<ALL>(sdf, g, at, c, v);
+  field_sum(c, v, lo);
+  field_load<ALL>(sdf, g, at + 1, c, v);
+  field_sum(c, v, hi);
+  for (int r = 0; r < rows; ++r, o += R) {
+    const int j0 = row_j0[r];
+    if (j0 != at) {
+      if (j0 == at + 1) {
+#pragma unroll
+        for (int p = 0; p < FIELD_NI; ++p) lo[p] = hi[p];
+      } else {
+        field_load<ALL>(sdf, g, j0, c, v);
+        field_sum(c, v, lo);
       }
-    float* orow = out + row * R;
-    for (int k = lane; k < R; k += 32) {
-      const float fk = world_to_index(g, 2, lattice(az, k, R));
-      const float fk0 = floorf(fk);
-      const int k0 = (int)fk0;
-      const float tk = fk - fk0;
-      const float wk[2] = {1.f - tk, tk};
-      float acc = 0.f;
+      field_load<ALL>(sdf, g, j0 + 1, c, v);
+      field_sum(c, v, hi);
+      at = j0;
+    }
+    const float2 wj = row_w[r];
 #pragma unroll
-      for (int di = 0; di < 2; ++di)
+    for (int p = 0; p < FIELD_NI; ++p)
+      if (p < n_i) __stcs(o + p * R * R, wj.x * lo[p] + wj.y * hi[p]);
+  }
+}
+
+__global__ void __launch_bounds__(FIELD_THREADS) sdf_field_kernel(const float* __restrict__ sdf, GridGeom g,
+                                                                  FieldAxis ax, FieldAxis ay, FieldAxis az, int R,
+                                                                  float sign, float* __restrict__ out) {
+  __shared__ float2 row_w[FIELD_ROWS];   // the rows' two y weights, times sign
+  __shared__ int row_j0[FIELD_ROWS];
+  const int ib = blockIdx.z * FIELD_NI, jb = blockIdx.y * FIELD_ROWS;
+  const int rows = min(FIELD_ROWS, R - jb), n_i = min(FIELD_NI, R - ib);
+  bool rows_in = true;
+  if ((int)threadIdx.x < rows) {
+    const float fj = world_to_index(g, 1, lattice(ay, jb + (int)threadIdx.x, R)), fj0 = floorf(fj);
+    const float tj = fj - fj0;
+    const int j0 = (int)fj0;
+    row_w[threadIdx.x] = make_float2(sign * (1.f - tj), sign * tj);
+    row_j0[threadIdx.x] = j0;
+    rows_in = j0 >= 0 && j0 < g.Y - 1;
+  }
+  rows_in = __syncthreads_and(rows_in);
+  const int k = blockIdx.x * FIELD_THREADS + threadIdx.x;
+  if (k >= R) return;
+  const float fk = world_to_index(g, 2, lattice(az, k, R)), fk0 = floorf(fk);
+  const int k0 = (int)fk0;
+  const float tk = fk - fk0;
+  FieldCols c;
+  c.wk[0] = 1.f - tk;
+  c.wk[1] = tk;
+  c.inside = 0;
 #pragma unroll
-        for (int dj = 0; dj < 2; ++dj)
+  for (int p = 0; p < FIELD_NI; ++p) {
+    const float fi = world_to_index(g, 0, lattice(ax, min(ib + p, R - 1), R)), fi0 = floorf(fi);
+    const int i0 = (int)fi0;
+    const float ti = fi - fi0;
+    c.wi[p][0] = 1.f - ti;
+    c.wi[p][1] = ti;
 #pragma unroll
-          for (int dk = 0; dk < 2; ++dk) {
-            const int kk = k0 + dk;
-            if (rin[di][dj] && kk >= 0 && kk < g.Z)
-              acc += (wi[di] * wj[dj] * wk[dk]) * __ldg(sdf + rbase[di][dj] + kk);
-          }
-      orow[k] = sign * acc;
+    for (int di = 0; di < 2; ++di) {
+      const int ii = i0 + di;
+      const bool in_i = ii >= 0 && ii < g.X;
+      c.col[p][di] = in_i ? ii * g.Y * g.Z + k0 : k0;
+#pragma unroll
+      for (int dk = 0; dk < 2; ++dk)
+        if (in_i && k0 + dk >= 0 && k0 + dk < g.Z) c.inside |= 1u << (4 * p + 2 * di + dk);
     }
   }
+  float* o = out + ((int64_t)ib * R + jb) * R + k;
+  const unsigned all = (1u << (4 * FIELD_NI)) - 1u;
+  if (rows_in && c.inside == all)
+    field_walk<true>(sdf, g, row_w, row_j0, rows, n_i, R, c, o);
+  else
+    field_walk<false>(sdf, g, row_w, row_j0, rows, n_i, R, c, o);
 }
 
 static FieldAxis field_axis(float start, float end, int64_t R) {
@@ -161,10 +239,9 @@ int vx_sdf_field(const float* sdf, const vx_grid_geom* grid, const float* bound_
   }
   const FieldAxis ax = field_axis(bound_min[0], bound_max[0], R), ay = field_axis(bound_min[1], bound_max[1], R),
                   az = field_axis(bound_min[2], bound_max[2], R);
-  const int64_t rows = R * R;  // one warp per row, 8 warps per block
-  const int64_t cap = (int64_t)sm_count() * 64;
-  const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((rows + 7) / 8, cap));
-  sdf_field_kernel<<<(unsigned)blocks, 256, 0, as_stream(stream)>>>(sdf, g, ax, ay, az, (int)R, sign, out);
+  const dim3 blocks((unsigned)((R + FIELD_THREADS - 1) / FIELD_THREADS), (unsigned)((R + FIELD_ROWS - 1) / FIELD_ROWS),
+                    (unsigned)((R + FIELD_NI - 1) / FIELD_NI));
+  sdf_field_kernel<<<blocks, FIELD_THREADS, 0, as_stream(stream)>>>(sdf, g, ax, ay, az, (int)R, sign, out);
   return launch_status();
 }
 
