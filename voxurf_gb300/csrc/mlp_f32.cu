@@ -23,9 +23,11 @@
 namespace vx {
 namespace mf {
 
-constexpr int BM = 64;       // rows per rowgemm tile
-constexpr int KC = 16;       // K per shared-memory stage
-constexpr int THREADS = 256; // 16 x 16 threads
+constexpr int BM = 64;          // rows per rowgemm tile
+constexpr int RG_THREADS = 128; // 8 x 16 threads
+constexpr int RG_M = BM / 8;    // rows per thread
+constexpr int KC = 16;          // K per shared-memory stage
+constexpr int THREADS = 256;    // weight gradient: 16 x 16 threads
 
 struct RowGemmParams {
   const float* A;            // [M, lda]
@@ -75,13 +77,18 @@ __device__ __forceinline__ void cp_wait_group() { asm volatile("cp.async.wait_gr
 constexpr int RG_STAGES = 3;   // shared-memory ring of the row GEMM
 constexpr int AS_LD = KC + 4;  // A stage row stride (floats): 16-byte rows, no bank conflicts
 
-// A 64-row tile of C = A Bt: each thread owns 4 rows x TN columns.  Stages of
-// KC columns of A ([64][KC] row-major) and KC rows of Bt ([KC][NP]) arrive by
-// cp.async in a three-deep ring, so the copies of the next two stages are in
-// flight while one is computed; A is read as float4 along k (one load per 4
-// k steps and row), Bt as float4 along n.
+// A 64-row tile of C = A Bt: each thread owns the rows ty + 8 i and TN
+// columns.  Stages of KC columns of A ([64][KC] row-major) and KC rows of Bt
+// ([KC][NP]) arrive by cp.async in a three-deep ring, so the copies of the next
+// two stages are in flight while one is computed; A is read as float4 along k
+// (one load per 4 k steps and row), Bt as float4 along n, and the products are
+// packed by column pairs (fma2: each half rounds as fmaf).
+// Bound: the FP32 pipes (73-77 TFLOP/s) while the shared-memory reads stay
+// below them: with 4 x 12 outputs a thread the reads of Bt took 81% of the L1
+// cycles.  131,003 rows: five layers (K = 70 and 192, N = 192) 1,039 us with
+// scalar products and 4 x 12 outputs a thread, 853 us now (57 TFLOP/s).
 template <int TN>
-__global__ void __launch_bounds__(THREADS, 2) rowgemm_kernel(RowGemmParams P) {
+__global__ void __launch_bounds__(RG_THREADS, 3) rowgemm_kernel(RowGemmParams P) {
   constexpr int NP = 16 * TN;
   // dynamic shared memory: the A ring, the Bt ring; the column-sum scratch of
   // the epilogue reuses the A ring
@@ -89,7 +96,7 @@ __global__ void __launch_bounds__(THREADS, 2) rowgemm_kernel(RowGemmParams P) {
   auto As = reinterpret_cast<float (*)[BM][AS_LD]>(rg_smem);
   auto Bs = reinterpret_cast<float (*)[KC][NP]>(rg_smem + RG_STAGES * BM * AS_LD);
   auto red = reinterpret_cast<float (*)[NP]>(rg_smem);
-  static_assert(16 * NP <= RG_STAGES * BM * AS_LD, "column-sum scratch fits the A ring");
+  static_assert(8 * NP <= RG_STAGES * BM * AS_LD, "column-sum scratch fits the A ring");
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   const int64_t M = rows_of(P.M, P.m_dev);
   const int64_t m0 = (int64_t)blockIdx.x * BM;
@@ -100,13 +107,16 @@ __global__ void __launch_bounds__(THREADS, 2) rowgemm_kernel(RowGemmParams P) {
   auto load_stage = [&](int kt, int slot) {
     const int k0 = kt * KC;
     if (avec) {
-      // 64 rows x 4 pieces of 16 bytes: one piece per thread
-      const int r = tid >> 2, c = 4 * (tid & 3);
-      const int64_t row = m0 + r;
-      const int valid = (row < M) ? max(0, min(4, P.K - (k0 + c))) : 0;
-      cp16(&As[slot][r][c], valid ? P.A + row * P.lda + k0 + c : P.A, (uint32_t)(4 * valid));
+      // 64 rows x 4 pieces of 16 bytes
+#pragma unroll
+      for (int i = tid; i < BM * 4; i += RG_THREADS) {
+        const int r = i >> 2, c = 4 * (i & 3);
+        const int64_t row = m0 + r;
+        const int valid = (row < M) ? max(0, min(4, P.K - (k0 + c))) : 0;
+        cp16(&As[slot][r][c], valid ? P.A + row * P.lda + k0 + c : P.A, (uint32_t)(4 * valid));
+      }
     } else {
-      for (int i = tid; i < BM * KC; i += THREADS) {
+      for (int i = tid; i < BM * KC; i += RG_THREADS) {
         const int r = i / KC, c = i % KC;
         const int64_t row = m0 + r;
         const bool ok = row < M && k0 + c < P.K;
@@ -115,14 +125,18 @@ __global__ void __launch_bounds__(THREADS, 2) rowgemm_kernel(RowGemmParams P) {
     }
     const float* src = P.Bt + (int64_t)kt * KC * NP;
     float* dst = &Bs[slot][0][0];
-    for (int i = tid; i < KC * NP / 4; i += THREADS) cp16(dst + 4 * i, src + 4 * i, 16u);
+    for (int i = tid; i < KC * NP / 4; i += RG_THREADS) cp16(dst + 4 * i, src + 4 * i, 16u);
   };
 
-  float acc[4][TN];
+  float acc[RG_M][TN];
+  f32x2 acc2[RG_M][TN % 4 == 0 ? TN / 2 : 1];   // pairs of columns (TN % 4 == 0)
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < RG_M; ++i)
 #pragma unroll
-    for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
+    for (int j = 0; j < TN; ++j) {
+      acc[i][j] = 0.f;
+      if constexpr (TN % 4 == 0) acc2[i][j / 2] = 0;
+    }
 
 #pragma unroll
   for (int s = 0; s < RG_STAGES - 1; ++s) {
@@ -137,33 +151,51 @@ __global__ void __launch_bounds__(THREADS, 2) rowgemm_kernel(RowGemmParams P) {
     const int slot = kt % RG_STAGES;
 #pragma unroll
     for (int k = 0; k < KC; k += 4) {
-      float a[4][4];
+      float a[RG_M][4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float4 v = *reinterpret_cast<const float4*>(&As[slot][4 * ty + i][k]);
+      for (int i = 0; i < RG_M; ++i) {
+        const float4 v = *reinterpret_cast<const float4*>(&As[slot][ty + 8 * i][k]);
         a[i][0] = v.x; a[i][1] = v.y; a[i][2] = v.z; a[i][3] = v.w;
       }
 #pragma unroll
       for (int kk = 0; kk < 4; ++kk) {
-        float b[TN];
         if constexpr (TN % 4 == 0) {
+          f32x2 b[TN / 2];
 #pragma unroll
           for (int j = 0; j < TN / 4; ++j) {
-            const float4 b4 = *reinterpret_cast<const float4*>(&Bs[slot][k + kk][TN * tx + 4 * j]);
-            b[4 * j] = b4.x; b[4 * j + 1] = b4.y; b[4 * j + 2] = b4.z; b[4 * j + 3] = b4.w;
+            const ulonglong2 b4 = *reinterpret_cast<const ulonglong2*>(&Bs[slot][k + kk][TN * tx + 4 * j]);
+            b[2 * j] = b4.x;
+            b[2 * j + 1] = b4.y;
+          }
+#pragma unroll
+          for (int i = 0; i < RG_M; ++i) {
+            const f32x2 aa = pack2(a[i][kk], a[i][kk]);
+#pragma unroll
+            for (int j = 0; j < TN / 2; ++j) acc2[i][j] = fma2(aa, b[j], acc2[i][j]);
           }
         } else {
+          float b[TN];
 #pragma unroll
           for (int j = 0; j < TN; ++j) b[j] = Bs[slot][k + kk][TN * tx + j];
+#pragma unroll
+          for (int i = 0; i < RG_M; ++i)
+#pragma unroll
+            for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i][kk], b[j], acc[i][j]);
         }
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i][kk], b[j], acc[i][j]);
       }
     }
   }
   cp_wait_group<0>();
+  if constexpr (TN % 4 == 0) {
+#pragma unroll
+    for (int i = 0; i < RG_M; ++i)
+#pragma unroll
+      for (int j = 0; j < TN / 2; ++j) {
+        const float2 v = unpack2(acc2[i][j]);
+        acc[i][2 * j] = v.x;
+        acc[i][2 * j + 1] = v.y;
+      }
+  }
   // epilogue
   float cs[TN];
 #pragma unroll
@@ -172,8 +204,8 @@ __global__ void __launch_bounds__(THREADS, 2) rowgemm_kernel(RowGemmParams P) {
   const bool cvec = (P.ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(P.C) & 15) == 0;
   const bool hvec = P.mode == 1 && (P.ldh & 3) == 0 && (reinterpret_cast<uintptr_t>(P.H) & 15) == 0;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int64_t m = m0 + 4 * ty + i;
+  for (int i = 0; i < RG_M; ++i) {
+    const int64_t m = m0 + ty + 8 * i;
     if (m >= M) continue;
     float v[TN];
 #pragma unroll
@@ -225,9 +257,9 @@ __global__ void __launch_bounds__(THREADS, 2) rowgemm_kernel(RowGemmParams P) {
 #pragma unroll
     for (int j = 0; j < TN; ++j) red[ty][n0 + j] = cs[j];
     __syncthreads();
-    for (int n = tid; n < NP; n += THREADS) {
+    for (int n = tid; n < NP; n += RG_THREADS) {
       float s = 0.f;
-      for (int r = 0; r < 16; ++r) s += red[r][n];
+      for (int r = 0; r < 8; ++r) s += red[r][n];
       P.colsum[(int64_t)blockIdx.x * NP + n] = s;
     }
   }
@@ -296,10 +328,14 @@ __global__ void __launch_bounds__(THREADS, 1) wgrad_kernel(WgradParams P) {
   };
 
   float acc[TM][TN];
+  f32x2 acc2[TM][TN % 4 == 0 ? TN / 2 : 1];   // pairs of columns (TN % 4 == 0)
 #pragma unroll
   for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
+    for (int j = 0; j < TN; ++j) {
+      acc[i][j] = 0.f;
+      if constexpr (TN % 4 == 0) acc2[i][j / 2] = 0;
+    }
   if (nst > 0) load(0, 0);
   cp_wait_all();
   __syncthreads();
@@ -308,18 +344,45 @@ __global__ void __launch_bounds__(THREADS, 1) wgrad_kernel(WgradParams P) {
     if (st + 1 < nst) load(st + 1, s ^ 1);   // lands while this stage is computed
 #pragma unroll 4
     for (int k = 0; k < WG_KC; ++k) {
-      float a[TM], b[TN];
+      float a[TM];
 #pragma unroll
       for (int i = 0; i < TM; ++i) a[i] = As[s][k][TM * ty + i];
+      if constexpr (TN % 4 == 0) {
+        f32x2 b[TN / 2];
 #pragma unroll
-      for (int j = 0; j < TN; ++j) b[j] = Bs[s][k][TN * tx + j];
+        for (int j = 0; j < TN / 4; ++j) {
+          const ulonglong2 b4 = *reinterpret_cast<const ulonglong2*>(&Bs[s][k][TN * tx + 4 * j]);
+          b[2 * j] = b4.x;
+          b[2 * j + 1] = b4.y;
+        }
 #pragma unroll
-      for (int i = 0; i < TM; ++i)
+        for (int i = 0; i < TM; ++i) {
+          const f32x2 aa = pack2(a[i], a[i]);
 #pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+          for (int j = 0; j < TN / 2; ++j) acc2[i][j] = fma2(aa, b[j], acc2[i][j]);
+        }
+      } else {
+        float b[TN];
+#pragma unroll
+        for (int j = 0; j < TN; ++j) b[j] = Bs[s][k][TN * tx + j];
+#pragma unroll
+        for (int i = 0; i < TM; ++i)
+#pragma unroll
+          for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+      }
     }
     cp_wait_all();
     __syncthreads();
+  }
+  if constexpr (TN % 4 == 0) {
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+      for (int j = 0; j < TN / 2; ++j) {
+        const float2 v = unpack2(acc2[i][j]);
+        acc[i][2 * j] = v.x;
+        acc[i][2 * j + 1] = v.y;
+      }
   }
   float* part = P.part + (size_t)blockIdx.x * MP * NP;
 #pragma unroll
@@ -423,7 +486,7 @@ int vx_mlp_f32_rowgemm(const vx_mlp_f32_rowgemm_args* a, void* stream) {
     const size_t smem = sizeof(float) * ((size_t)RG_STAGES * BM * AS_LD + (size_t)RG_STAGES * KC * np);
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return cuda_status(e);
-    kernel<<<grid, THREADS, smem, st>>>(P);
+    kernel<<<grid, RG_THREADS, smem, st>>>(P);
     return launch_status();
   };
   switch (a->Np) {
