@@ -1,9 +1,12 @@
-// Colour-MLP training in plain FP32 on the CUDA cores: the hidden layers of
-// rgbnet / k_rgbnet (lib/voxurf_fine.py:132-187) and of the coarse rgbnet
+// Colour-MLP training in plain FP32: the hidden layers of rgbnet / k_rgbnet
+// (lib/voxurf_fine.py:132-187) and of the coarse rgbnet
 // (lib/voxurf_coarse.py:116-123), forward and backward, with FP32 operands
-// and FP32 fused multiply-adds (the arithmetic of the reference's FP32
-// nn.Linear under autograd).  The 3-wide output layer has kernels of its own
-// (vx_mlp_head, vx_mlp_head_backward in mlp_ops.cu).
+// and FP32 fused multiply-adds on the CUDA cores (the arithmetic of the
+// reference's FP32 nn.Linear under autograd).  The backward GEMMs of 128- and
+// 192-wide layers with aligned rows run on the tensor cores with split
+// operands (mlp_f32_split.cu); the kernels here take the forward and what is
+// left.  The 3-wide output layer has kernels of its own (vx_mlp_head,
+// vx_mlp_head_backward in mlp_ops.cu).
 //
 //   rowgemm_kernel   C[m][n] = sum_k A[m][k] Bt[k][n] over a 64-row tile and
 //                    all N columns (N = 16 TN), with one of three epilogues:
@@ -18,7 +21,7 @@
 //                    fixed order.
 #include <algorithm>
 
-#include "common.cuh"
+#include "mlp_f32.cuh"
 
 namespace vx {
 namespace mf {
@@ -28,24 +31,6 @@ constexpr int RG_THREADS = 128; // 8 x 16 threads
 constexpr int RG_M = BM / 8;    // rows per thread
 constexpr int KC = 16;          // K per shared-memory stage
 constexpr int THREADS = 256;    // weight gradient: 16 x 16 threads
-
-struct RowGemmParams {
-  const float* A;            // [M, lda]
-  int64_t lda;
-  int64_t M;
-  const int64_t* m_dev;      // optional device row count (<= M)
-  int K;                     // columns of A used
-  const float* Bt;           // [Kp][Np] (Kp = round_up(K, 16), zero rows beyond K)
-  int Np;
-  int mode;                  // 0: relu(acc + bias); 1: acc * [H > 0] + column sums; 2: acc
-  const float* bias;         // mode 0: [Np]
-  const float* H;            // mode 1: [M, ldh] post-ReLU activation of the layer
-  int64_t ldh;
-  float* C;                  // [M, ldc], columns < n_store
-  int64_t ldc;
-  int n_store;
-  float* colsum;             // mode 1: [gridDim.x][Np] per-CTA column sums
-};
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
@@ -57,14 +42,6 @@ __device__ __forceinline__ void cp16(void* dst, const void* src, uint32_t src_by
 }
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-
-__device__ __forceinline__ int64_t rows_of(int64_t n, const int64_t* n_dev) {
-  if (n_dev) {
-    const int64_t d = *n_dev;
-    if (d < n) n = d < 0 ? 0 : d;
-  }
-  return n;
-}
 
 // 4-byte asynchronous copy (rows whose stride is not a multiple of 4 floats).
 __device__ __forceinline__ void cp4(void* dst, const void* src, uint32_t src_bytes) {
@@ -266,17 +243,6 @@ __global__ void __launch_bounds__(RG_THREADS, 3) rowgemm_kernel(RowGemmParams P)
 }
 
 // ---------------------------------------------------------------------------
-struct WgradParams {
-  const float* A;            // [rows, lda] (dz of the layer's output), columns < M
-  int64_t lda;
-  const float* B;            // [rows, ldb] (the layer's input), columns < N
-  int64_t ldb;
-  int M, N;                  // N <= 16 TN, M <= 16 TM
-  int64_t rows;
-  const int64_t* rows_dev;
-  float* part;               // [gridDim.x][16 TM][16 TN]
-};
-
 constexpr int WG_KC = 16;    // rows per stage
 
 template <int TM, int TN>
@@ -328,14 +294,10 @@ __global__ void __launch_bounds__(THREADS, 1) wgrad_kernel(WgradParams P) {
   };
 
   float acc[TM][TN];
-  f32x2 acc2[TM][TN % 4 == 0 ? TN / 2 : 1];   // pairs of columns (TN % 4 == 0)
 #pragma unroll
   for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int j = 0; j < TN; ++j) {
-      acc[i][j] = 0.f;
-      if constexpr (TN % 4 == 0) acc2[i][j / 2] = 0;
-    }
+    for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
   if (nst > 0) load(0, 0);
   cp_wait_all();
   __syncthreads();
@@ -344,45 +306,18 @@ __global__ void __launch_bounds__(THREADS, 1) wgrad_kernel(WgradParams P) {
     if (st + 1 < nst) load(st + 1, s ^ 1);   // lands while this stage is computed
 #pragma unroll 4
     for (int k = 0; k < WG_KC; ++k) {
-      float a[TM];
+      float a[TM], b[TN];
 #pragma unroll
       for (int i = 0; i < TM; ++i) a[i] = As[s][k][TM * ty + i];
-      if constexpr (TN % 4 == 0) {
-        f32x2 b[TN / 2];
 #pragma unroll
-        for (int j = 0; j < TN / 4; ++j) {
-          const ulonglong2 b4 = *reinterpret_cast<const ulonglong2*>(&Bs[s][k][TN * tx + 4 * j]);
-          b[2 * j] = b4.x;
-          b[2 * j + 1] = b4.y;
-        }
+      for (int j = 0; j < TN; ++j) b[j] = Bs[s][k][TN * tx + j];
 #pragma unroll
-        for (int i = 0; i < TM; ++i) {
-          const f32x2 aa = pack2(a[i], a[i]);
+      for (int i = 0; i < TM; ++i)
 #pragma unroll
-          for (int j = 0; j < TN / 2; ++j) acc2[i][j] = fma2(aa, b[j], acc2[i][j]);
-        }
-      } else {
-        float b[TN];
-#pragma unroll
-        for (int j = 0; j < TN; ++j) b[j] = Bs[s][k][TN * tx + j];
-#pragma unroll
-        for (int i = 0; i < TM; ++i)
-#pragma unroll
-          for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-      }
+        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
     }
     cp_wait_all();
     __syncthreads();
-  }
-  if constexpr (TN % 4 == 0) {
-#pragma unroll
-    for (int i = 0; i < TM; ++i)
-#pragma unroll
-      for (int j = 0; j < TN / 2; ++j) {
-        const float2 v = unpack2(acc2[i][j]);
-        acc[i][2 * j] = v.x;
-        acc[i][2 * j + 1] = v.y;
-      }
   }
   float* part = P.part + (size_t)blockIdx.x * MP * NP;
 #pragma unroll
@@ -480,8 +415,10 @@ int vx_mlp_f32_rowgemm(const vx_mlp_f32_rowgemm_args* a, void* stream) {
   P.ldc = a->ldc;
   P.n_store = (int)a->n_store;
   P.colsum = a->colsum;
+  P.n_colsum = (int64_t)vx_mlp_f32_rowgemm_grid(a->M);
   const unsigned grid = (unsigned)vx_mlp_f32_rowgemm_grid(a->M);
   cudaStream_t st = as_stream(stream);
+  if (split_rowgemm_takes(P)) return split_rowgemm_launch(P, st);
   auto launch = [&](auto kernel, int np) -> int {
     const size_t smem = sizeof(float) * ((size_t)RG_STAGES * BM * AS_LD + (size_t)RG_STAGES * KC * np);
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -523,6 +460,7 @@ int vx_mlp_f32_wgrad(const vx_mlp_f32_wgrad_args* a, void* stream) {
   P.rows_dev = a->rows_dev;
   P.part = a->part;
   cudaStream_t st = as_stream(stream);
+  if (split_wgrad_takes(P, (int)MP, (int)NP)) return split_wgrad_launch(P, (int)MP, (int)NP, grid, st);
 #define VX_WG(TM_, TN_)                                            \
   if (MP == 16 * TM_ && NP == 16 * TN_) {                          \
     wgrad_kernel<TM_, TN_><<<grid, THREADS, 0, st>>>(P);           \

@@ -7,7 +7,9 @@ Two native engines, both hand-written sm_103a kernels:
 * BF16 rows (the mixed-precision path): TcTrainMLP, the tcgen05 tensor-core
   kernels of mlp_train.cu (BF16 operands, FP32 accumulation);
 * FP32 rows (the plain path): F32TrainMLP, FP32 CUDA-core kernels
-  (mlp_f32.cu) for the hidden layers and the fused output-layer kernels of
+  (mlp_f32.cu) for the hidden layers' forward, their backward on the tensor
+  cores with every FP32 operand in three BF16 parts (mlp_f32_split.cu, no less
+  exact than the CUDA-core sums), and the fused output-layer kernels of
   mlp_ops.cu (vx_mlp_head, vx_mlp_head_backward).
 Parameters stay FP32 masters (the reference's nn.Linear parameters, same
 names and shapes); each forward refreshes the engine's operand copies of
@@ -111,8 +113,8 @@ def last_relu_masks(net: nn.Sequential) -> list[torch.Tensor] | None:
 
 
 class F32TrainMLP:
-    """Plain-FP32 engine: the hidden layers as FP32 CUDA-core GEMMs with
-    fused epilogues (vx_mlp_f32_rowgemm: +bias and ReLU forward; ReLU mask and
+    """Plain-FP32 engine: the hidden layers as FP32 GEMMs with fused
+    epilogues (vx_mlp_f32_rowgemm: +bias and ReLU forward; ReLU mask and
     bias-gradient column sums backward), their weight gradients summed over
     rows per CTA (vx_mlp_f32_wgrad) and in a fixed order (vx_mlp_f32_reduce),
     the 3-wide output layer in vx_mlp_head / vx_mlp_head_backward."""
