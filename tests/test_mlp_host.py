@@ -1,0 +1,34 @@
+"""Host logic of the MLP engines: the module and parameter lists they walk."""
+import gc
+
+import torch.nn as nn
+
+from voxurf_gb300.mlp import _linears, _modules, _parameters
+
+
+def _stacks():
+    shared = nn.Linear(4, 4)
+    yield nn.Sequential(nn.Linear(3, 4), nn.ReLU(), nn.Sequential(nn.Linear(4, 4), nn.ReLU()), nn.Linear(4, 3))
+    yield nn.Sequential(shared, nn.Sequential(nn.Linear(4, 4, bias=False), shared, nn.ReLU()), nn.Linear(4, 3))
+    yield nn.Linear(2, 3)
+
+
+def test_walks_equal_torch():
+    for net in _stacks():
+        assert [id(m) for m in _modules(net)] == [id(m) for m in net.modules()]
+        assert [id(p) for p in _parameters(net)] == [id(p) for p in net.parameters()]
+        assert [id(m) for m in _linears(net)] == [id(m) for m in net.modules() if isinstance(m, nn.Linear)]
+
+
+def test_walks_leave_no_cycles():
+    """A cycle per call would hold the modules until the collector runs, which
+    may be in the middle of a stream capture."""
+    net = next(_stacks())
+    gc.collect()
+    gc.disable()
+    try:
+        for _ in range(10):
+            _linears(net), _parameters(net)
+        assert gc.collect() == 0
+    finally:
+        gc.enable()

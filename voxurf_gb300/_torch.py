@@ -15,6 +15,14 @@ def ptr(t: torch.Tensor | None) -> int | None:
 
 
 def stream_ptr(device: torch.device | None = None) -> int:
+    """The current CUDA stream of `device` (default: the current device).
+    The raw handle takes under a microsecond; torch.cuda.current_stream builds
+    a Stream object for it, which cost more than a small kernel per call."""
+    if device is None or (type(device) is torch.device and device.type == "cuda"):
+        if not torch.cuda.is_initialized():
+            torch.cuda.init()
+        index = None if device is None else device.index
+        return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice() if index is None else index)
     return torch.cuda.current_stream(device).cuda_stream
 
 

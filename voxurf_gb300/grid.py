@@ -39,7 +39,7 @@ def host_values(t: torch.Tensor) -> list:
     """Host copy of a small device tensor (bbox, mask scale/shift), cached
     per tensor storage and version: a per-step .tolist() would make the host
     wait for all queued GPU work of the previous step."""
-    key = (t.data_ptr(), t._version, tuple(t.shape), str(t.device))
+    key = (t.data_ptr(), t._version, t.shape, t.device)
     hit = _HOST_CACHE.get(id(t))
     if hit is not None and hit[0] == key:
         return hit[1]

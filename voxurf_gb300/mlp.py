@@ -66,13 +66,15 @@ class _TrainMLP(torch.autograd.Function):
 _ENGINES: "weakref.WeakKeyDictionary[nn.Module, dict]" = weakref.WeakKeyDictionary()
 
 
-def engine_for(net: nn.Sequential, dtype: torch.dtype, ld: int):
+def engine_for(net: nn.Sequential, dtype: torch.dtype, ld: int, lin: list | None = None):
     """The engine of `net` for input rows of `dtype` with row stride `ld`
-    (cached per module; its operand buffers follow the parameters)."""
+    (cached per module; its operand buffers follow the parameters).  lin:
+    _linears(net), where the caller has it."""
     cache = _ENGINES.setdefault(net, {})
     key = (dtype, ld)
     eng = cache.get(key)
-    lin = _linears(net)
+    if lin is None:
+        lin = _linears(net)
     if eng is None or eng.lin[0].weight.data_ptr() != lin[0].weight.data_ptr():
         eng = TcTrainMLP(net, ld) if dtype == torch.bfloat16 else F32TrainMLP(net)
         cache[key] = eng
@@ -93,8 +95,8 @@ def apply_mlp(net: nn.Sequential, x: torch.Tensor, cols: torch.Tensor | None = N
     if x.dtype == torch.bfloat16 and ld % 16:
         ld = _round_up(ld, 16)
         x = torch.nn.functional.pad(x, (0, ld - x.shape[1]))
-    eng = engine_for(net, x.dtype, ld)
-    return _TrainMLP.apply(x, eng, cols, *net.parameters())
+    eng = engine_for(net, x.dtype, ld, lin)
+    return _TrainMLP.apply(x, eng, cols, *_parameters(net))
 
 
 def mlp_params(net: nn.Sequential) -> list[torch.Tensor]:
@@ -156,10 +158,7 @@ class F32TrainMLP:
         _abi.call("vx_mlp_train_pack", self.jobs, len(self.jobs), stream_ptr(self.device) if stream is None else stream)
 
     def grad_buffers(self) -> list[torch.Tensor]:
-        out = []
-        for m in self.lin:
-            out += [torch.empty_like(m.weight), torch.empty_like(m.bias)]
-        return out
+        return _grad_buffers(self.lin)
 
     def _rowgemm(self, mode, A, K, Bt, Np, C, n_store, bias=None, H=None, colsum=None, n_rows_dev=None):
         from . import _abi
@@ -222,8 +221,7 @@ class F32TrainMLP:
             dX = torch.empty((n, X.shape[1]), dtype=torch.float32, device=dev)
         # the output-layer kernel accumulates dWh, dbh and db_{L-1}
         dWh, dbh, dbL = grads[2 * L], grads[2 * L + 1], grads[2 * (L - 1) + 1]
-        for t in (dWh, dbh, dbL):
-            t.zero_()
+        torch._foreach_zero_([dWh, dbh, dbL])
         lh = self.lin[-1]
         dz = w["dz"][0]
         call("vx_mlp_head_backward", ptr(dY), ptr(hs[-1]), lh.weight.data_ptr(), n, W, 0, ptr(dz), ptr(dWh),
@@ -314,8 +312,57 @@ class TensorCoreMLP:
         _abi.call_struct("vx_mlp_tc_forward", a, stream_ptr(X.device))
 
 
-def _linears(net: nn.Sequential) -> list:
-    return [m for m in net.modules() if isinstance(m, nn.Linear)]
+def _modules(net: nn.Module) -> list:
+    """net.modules() as a list, in its order and each module once (the
+    generator of nn.Module costs ten times as much on these small stacks)."""
+    out, todo = [], [net]
+    while todo:
+        m = todo.pop()
+        if not any(m is o for o in out):
+            out.append(m)
+            todo.extend(c for c in reversed(m._modules.values()) if c is not None)
+    return out
+
+
+def _linears(net: nn.Module) -> list:
+    return [m for m in _modules(net) if isinstance(m, nn.Linear)]
+
+
+def _parameters(net: nn.Module) -> list:
+    """net.parameters() as a list, in its order and each parameter once."""
+    out = []
+    for m in _modules(net):
+        for p in m._parameters.values():
+            if p is not None and not any(p is o for o in out):
+                out.append(p)
+    return out
+
+
+def _grad_buffers(lin: list) -> list[torch.Tensor]:
+    """FP32 gradient buffers [W0, b0, ..., Wh, bh] of Linear layers, parts of
+    one allocation."""
+    shapes = []
+    for m in lin:
+        shapes += [m.weight.shape, m.bias.shape]
+    flat = torch.empty(sum(s.numel() for s in shapes), dtype=torch.float32, device=lin[0].weight.device)
+    return [t if len(s) == 1 else t.view(s) for t, s in zip(flat.split([s.numel() for s in shapes]), shapes)]
+
+
+class _Scratch:
+    """One allocation for several buffers of an engine: `take` hands out
+    256-byte aligned offsets, `alloc` makes the bytes.  Seven torch.empty calls
+    cost more host time than the kernels of a small batch."""
+
+    def __init__(self):
+        self.nbytes = 0
+
+    def take(self, nbytes: int) -> int:
+        at = self.nbytes
+        self.nbytes = _round_up(at + nbytes, 256)
+        return at
+
+    def alloc(self, device) -> torch.Tensor:
+        return torch.empty(max(self.nbytes, 16), dtype=torch.uint8, device=device)
 
 
 class TcTrainMLP:
@@ -398,10 +445,7 @@ class TcTrainMLP:
 
     def grad_buffers(self) -> list[torch.Tensor]:
         """FP32 gradient buffers in parameter order [W0, b0, ..., Wh, bh]."""
-        out = []
-        for m in self.lin:
-            out += [torch.empty_like(m.weight), torch.empty_like(m.bias)]
-        return out
+        return _grad_buffers(self.lin)
 
     def forward(self, X: torch.Tensor, out: torch.Tensor | None = None, train: bool = True,
                 cols: torch.Tensor | None = None, n_rows_dev: torch.Tensor | None = None,
@@ -422,9 +466,10 @@ class TcTrainMLP:
         st = None
         if train:
             st = saved if saved is not None else {}
-            if "H" not in st:
-                st["H"] = torch.empty(self.L * cap * self.W, dtype=torch.bfloat16, device=dev)
-                st["relu"] = torch.empty(self.L * cap * (self.W // 16), dtype=torch.int16, device=dev)
+            if "buf" not in st:
+                sc = _Scratch()
+                st["at"] = (sc.take(self.L * cap * self.W * 2), sc.take(self.L * cap * (self.W // 16) * 2))
+                st["buf"] = sc.alloc(dev)   # hidden T-tiles, ReLU bits
             st["cap"], st["n"], st["X"], st["n_rows_dev"] = cap, n, X, n_rows_dev
         a = _abi.MlpTrainFwdArgs()
         a.n_rows, a.n_rows_dev, a.rows_cap = n, ptr(n_rows_dev), cap
@@ -436,7 +481,7 @@ class TcTrainMLP:
             raise ValueError("cols must be BF16 for BF16 rows")
         a.cols, a.ld_cols = ptr(cols), (cols.stride(0) if cols is not None else 0)
         if train:
-            a.H, a.relu = ptr(st["H"]), ptr(st["relu"])
+            a.H, a.relu = (st["buf"].data_ptr() + o for o in st["at"])
         _abi.call_struct("vx_mlp_train_forward", a, stream_ptr(dev))
         return out, st
 
@@ -467,13 +512,15 @@ class TcTrainMLP:
             raise ValueError("dY must be contiguous FP32 [n, 3]")
         grid = int(lib.vx_mlp_wgrad_grid(n))
         w = work if work is not None else {}
-        if "dZ" not in w:
-            w["dZ"] = torch.empty(L * cap * W, dtype=torch.bfloat16, device=dev)
-            w["dYT"] = torch.empty(cap * 16, dtype=torch.bfloat16, device=dev)
-            w["dbh"] = torch.empty(grid * 4, dtype=torch.float32, device=dev)
-            w["part"] = [torch.empty(grid * W * (W + 16), dtype=torch.float32, device=dev) for _ in range(L - 1)]
-            w["part0"] = torch.empty(grid * W * (K0 + 16), dtype=torch.float32, device=dev)
-            w["parth"] = torch.empty(grid * W * 16, dtype=torch.float32, device=dev)
+        if "buf" not in w:
+            # dz T-tiles, dy T-tiles, column sums of dy, weight-gradient partials
+            sc = _Scratch()
+            offs = [sc.take(L * cap * W * 2), sc.take(cap * 16 * 2), sc.take(grid * 4 * 4),
+                    sc.take(grid * W * (K0 + 16) * 4), sc.take(grid * W * 16 * 4)]
+            offs += [sc.take(grid * W * (W + 16) * 4) for _ in range(L - 1)]
+            w["buf"], w["at"] = sc.alloc(dev), offs
+        dZ, dYT, dbh, part0, parth, *part = (w["buf"].data_ptr() + o for o in w["at"])
+        H, relu = (st["buf"].data_ptr() + o for o in st["at"])
         if dX is None:
             dX = torch.empty((n, K0), dtype=dx_dtype, device=dev)
         if grads is None:
@@ -481,33 +528,32 @@ class TcTrainMLP:
         b = _abi.MlpTrainBwdArgs()
         b.n_rows, b.n_rows_dev, b.rows_cap = n, ptr(st["n_rows_dev"]), cap
         b.width, b.n_hidden, b.K0 = W, L, K0
-        b.dY, b.Wh, b.relu = ptr(dY), self.lin[-1].weight.data_ptr(), ptr(st["relu"])
-        b.WTp, b.W0Tp, b.dZ, b.dYT = ptr(self.WTp), ptr(self.W0Tp), ptr(w["dZ"]), ptr(w["dYT"])
+        b.dY, b.Wh, b.relu = ptr(dY), self.lin[-1].weight.data_ptr(), relu
+        b.WTp, b.W0Tp, b.dZ, b.dYT = ptr(self.WTp), ptr(self.W0Tp), dZ, dYT
         b.dX, b.ld_dx, b.dx_bf16 = ptr(dX), dX.stride(0), int(dX.dtype == torch.bfloat16)
-        b.dbh_part, b.dbh_part_cap = ptr(w["dbh"]), grid
+        b.dbh_part, b.dbh_part_cap = dbh, grid
         _abi.call_struct("vx_mlp_train_backward", b, stp)
-        H, dZ = st["H"].data_ptr(), w["dZ"].data_ptr()
         lay = cap * W * 2   # bytes per layer of T-tiles
         R = _abi.MlpReduceJob
-        pending = []   # (pass arguments, reduce job of its n_part partials)
+        pending = []   # (pass arguments, reduce job of its n_part partials, the buffers both point into)
 
         def wgrad(A, WA, B, WB, ldb, b_rows, ones, part, job):
             g = _abi.MlpWgradArgs()
             g.n_rows, g.n_rows_dev, g.A, g.WA, g.B, g.WB, g.ldb = n, ptr(st["n_rows_dev"]), A, WA, B, WB, ldb
-            g.b_rows, g.ones, g.part, g.part_cap = b_rows, ones, ptr(part), part.numel()
-            pending.append((g, job))
+            g.b_rows, g.ones, g.part, g.part_cap = b_rows, ones, part, grid * WA * (WB + 16 * ones)
+            pending.append((g, job, (w["buf"], st["buf"], X)))
 
         for l in range(1, L):   # dW_l = dz_{l+1}^T h_l
-            pl = w["part"][l - 1]
+            pl = part[l - 1]
             wgrad(dZ + l * lay, W, H + (l - 1) * lay, W, 0, 0, 1, pl,
-                  lambda k, pl=pl, l=l: R(pl.data_ptr(), k, W, W + 16, 0, 0, W, W, grads[2 * l].data_ptr(),
+                  lambda k, pl=pl, l=l: R(pl, k, W, W + 16, 0, 0, W, W, grads[2 * l].data_ptr(),
                                           grads[2 * l + 1].data_ptr(), None, 0))
-        wgrad(dZ, W, X.data_ptr(), K0, X.stride(0), 1, 1, w["part0"],      # dW_0 = dz_1^T X
-              lambda k: R(w["part0"].data_ptr(), k, W, K0 + 16, 0, 0, K0, self.d_in, grads[0].data_ptr(),
+        wgrad(dZ, W, X.data_ptr(), K0, X.stride(0), 1, 1, part0,      # dW_0 = dz_1^T X
+              lambda k: R(part0, k, W, K0 + 16, 0, 0, K0, self.d_in, grads[0].data_ptr(),
                           grads[1].data_ptr(), None, 0))
-        wgrad(H + (L - 1) * lay, W, w["dYT"].data_ptr(), 16, 0, 0, 0, w["parth"],   # dWh = dy^T h_L
-              lambda k: R(w["parth"].data_ptr(), k, W, 16, 1, 0, 16, 3, grads[2 * L].data_ptr(),
-                          grads[2 * L + 1].data_ptr(), w["dbh"].data_ptr(), grid))
+        wgrad(H + (L - 1) * lay, W, dYT, 16, 0, 0, 0, parth,   # dWh = dy^T h_L
+              lambda k: R(parth, k, W, 16, 1, 0, 16, 3, grads[2 * L].data_ptr(),
+                          grads[2 * L + 1].data_ptr(), dbh, grid))
         return dX, grads, pending
 
     @staticmethod
@@ -525,10 +571,10 @@ class TcTrainMLP:
         for i in range(0, len(items), 8):
             grp = items[i:i + 8]
             k = len(grp)
-            arr = (_abi.MlpWgradArgs * k)(*[g for g, _ in grp])
+            arr = (_abi.MlpWgradArgs * k)(*[g for g, _, _ in grp])
             ctas = (ctypes.c_int32 * k)()
             _native.check(lib.vx_mlp_wgrad_split(arr, k, ctas), "vx_mlp_wgrad_split")
             _native.check(lib.vx_mlp_train_wgrad_multi(arr, ctas, k, stream), "vx_mlp_train_wgrad_multi")
-            jobs = [mk(int(ctas[j])) for j, (_, mk) in enumerate(grp)]
+            jobs = [mk(int(ctas[j])) for j, (_, mk, _) in enumerate(grp)]
             _abi.call("vx_mlp_train_reduce", (_abi.MlpReduceJob * k)(*jobs), k, stream)
 

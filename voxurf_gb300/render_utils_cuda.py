@@ -111,7 +111,7 @@ def maskcache_lookup(world, xyz, xyz2ijk_scale, xyz2ijk_shift):
     if world.dim() != 3 or xyz.dim() != 2 or xyz.size(1) != 3:
         raise RuntimeError("world must be [X,Y,Z] and xyz [M,3]")
     n = xyz.size(0)
-    out = torch.zeros(n, dtype=torch.bool, device=xyz.device)
+    out = torch.empty(n, dtype=torch.bool, device=xyz.device)   # the kernel writes every point
     if n == 0:
         return out
     call("vx_maskcache_lookup", ptr(world), world.size(0), world.size(1), world.size(2), ptr(xyz), n,
