@@ -815,6 +815,9 @@ typedef struct {
 } vx_mlp_f32_rowgemm_args;
 
 size_t vx_mlp_f32_rowgemm_grid(int64_t M);
+/* Leading rows of colsum that a mode 1 call with these arguments fills with
+ * sums; the others are written as zeros. */
+size_t vx_mlp_f32_colsum_rows(const vx_mlp_f32_rowgemm_args* args);
 /* C = A Bt with the epilogue of `mode` (lib/voxurf_fine.py:132-151 forward,
  * and its autograd backward). */
 int vx_mlp_f32_rowgemm(const vx_mlp_f32_rowgemm_args* args, void* stream);

@@ -61,6 +61,7 @@ def test_rowgemm_is_exact_on_integers(cuda, mode, K, Np, n_store, pad, M):
     elif mode == 1:
         ref = ref * (H[:m, :Np] > 0)
         assert torch.equal(colsum.view(-1, Np).double().sum(0), ref.sum(0))
+        assert bool((colsum.view(-1, Np)[int(lib.vx_mlp_f32_colsum_rows(g)):] == 0).all())
     assert torch.equal(C[:m, :n_store].double(), ref[:, :n_store])
     assert bool((C[m:] == 7).all()) and bool((C[:, n_store:] == 7).all())
     assert _native.device_error(stream_ptr(cuda)) == 0

@@ -335,6 +335,8 @@ def _declare():
     lib.vx_mlp_wgrad_grid.restype = C.c_size_t
     lib.vx_mlp_f32_rowgemm_grid.argtypes = [I64]
     lib.vx_mlp_f32_rowgemm_grid.restype = C.c_size_t
+    lib.vx_mlp_f32_colsum_rows.argtypes = [C.POINTER(MlpF32RowGemmArgs)]
+    lib.vx_mlp_f32_colsum_rows.restype = C.c_size_t
     lib.vx_mlp_f32_wgrad_grid.argtypes = [I64]
     lib.vx_mlp_f32_wgrad_grid.restype = C.c_size_t
     lib.vx_mlp_f32_reduce.argtypes = [C.POINTER(MlpSumJob), C.c_int, P]
@@ -391,7 +393,7 @@ def struct_names() -> list[str]:
                                 "vx_smooth_grad_tv_scratch_bytes", "vx_smooth_grad_tv",
                                 "vx_sdf_field", "vx_density_mask", "vx_hit_coarse_geo", "vx_bg_samples_count",
                                 "vx_bg_samples_fill", "vx_cast_rows_bf16", "vx_mlp_train_pack",
-                                "vx_mlp_train_reduce", "vx_mlp_wgrad_grid", "vx_mlp_train_wgrad_multi", "vx_mlp_wgrad_split", "vx_mlp_f32_rowgemm_grid",
+                                "vx_mlp_train_reduce", "vx_mlp_wgrad_grid", "vx_mlp_train_wgrad_multi", "vx_mlp_wgrad_split", "vx_mlp_f32_rowgemm_grid", "vx_mlp_f32_colsum_rows",
                                 "vx_mlp_f32_wgrad_grid", "vx_mlp_f32_reduce",
                                 "vx_fine_composite_loss_scratch_bytes", "vx_tv_loss_scratch_bytes", "vx_tv_loss",
                                 "vx_tv_loss_backward"] + list(_SERVE_SIGNATURES)

@@ -22,7 +22,7 @@ struct RowGemmParams {
   int64_t ldc;
   int n_store;
   float* colsum;             // mode 1: [n_colsum][Np] column sums, one row per CTA
-  int64_t n_colsum;          // vx_mlp_f32_rowgemm_grid(M) rows, each written
+  int64_t n_colsum;          // vx_mlp_f32_rowgemm_grid(M) rows, those beyond the CTAs zero
 };
 
 struct WgradParams {
@@ -47,6 +47,7 @@ __device__ __forceinline__ int64_t rows_of(int64_t n, const int64_t* n_dev) {
 // The backward GEMMs on the tensor cores; false when the shapes or the
 // alignment of the buffers are not theirs (the CUDA-core kernels run then).
 bool split_rowgemm_takes(const RowGemmParams& P);
+unsigned split_rowgemm_grid(int64_t M);
 int split_rowgemm_launch(const RowGemmParams& P, cudaStream_t st);
 bool split_wgrad_takes(const WgradParams& P, int MP, int NP);
 int split_wgrad_launch(const WgradParams& P, int MP, int NP, unsigned grid, cudaStream_t st);

@@ -370,15 +370,17 @@ bool split_rowgemm_takes(const RowGemmParams& P) {
          a16 % 16 == 0 && c8 % 8 == 0 && P.ldc % 2 == 0 && (P.mode != 1 || (P.ldh % 2 == 0 && P.n_store == P.Np));
 }
 
+unsigned split_rowgemm_grid(int64_t M) {
+  return (unsigned)std::min<int64_t>(std::max<int64_t>(1, (M + TILE_M - 1) / TILE_M), sm_count());
+}
+
 template <int K, int N>
 static int rowgemm_go(const RowGemmParams& P, cudaStream_t st) {
   using G = RowGemmGeo<K, N>;
   const cudaError_t e =
       cudaFuncSetAttribute(split_rowgemm_kernel<K, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::SMEM);
   if (e != cudaSuccess) return cuda_status(e);
-  const int64_t tiles = std::max<int64_t>(1, (P.M + TILE_M - 1) / TILE_M);
-  const unsigned grid = (unsigned)std::min<int64_t>(tiles, sm_count());
-  split_rowgemm_kernel<K, N><<<grid, SP_THREADS, G::SMEM, st>>>(P, device_error_ptr());
+  split_rowgemm_kernel<K, N><<<split_rowgemm_grid(P.M), SP_THREADS, G::SMEM, st>>>(P, device_error_ptr());
   return launch_status();
 }
 

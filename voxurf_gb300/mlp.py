@@ -170,6 +170,7 @@ class F32TrainMLP:
         g.C, g.ldc, g.n_store = ptr(C), C.stride(0), n_store
         g.colsum, g.colsum_cap = ptr(colsum), 0 if colsum is None else colsum.numel()
         _abi.call_struct("vx_mlp_f32_rowgemm", g, stream_ptr(A.device))
+        return g
 
     def forward(self, X: torch.Tensor, out: torch.Tensor | None = None, train: bool = True,
                 cols: torch.Tensor | None = None, n_rows_dev: torch.Tensor | None = None,
@@ -239,8 +240,8 @@ class F32TrainMLP:
             wgrad(dz, hs[l - 1], W, w["part"][l - 1])
             sums.append(S(w["part"][l - 1].data_ptr(), g_wg, W * W, W, W, W, grads[2 * l].data_ptr(), W))
             nxt = w["dz"][(L - l) % 2]
-            self._rowgemm(1, dz, W, self.Bb[l], W, nxt, W, H=hs[l - 1], colsum=w["colsum"][l - 1], n_rows_dev=nrd)
-            sums.append(S(w["colsum"][l - 1].data_ptr(), g_rows, W, W, 1, W, grads[2 * (l - 1) + 1].data_ptr(), W))
+            g = self._rowgemm(1, dz, W, self.Bb[l], W, nxt, W, H=hs[l - 1], colsum=w["colsum"][l - 1], n_rows_dev=nrd)
+            sums.append(S(w["colsum"][l - 1].data_ptr(), int(lib.vx_mlp_f32_colsum_rows(g)), W, W, 1, W, grads[2 * (l - 1) + 1].data_ptr(), W))
             dz = nxt
         wgrad(dz, X, self.d_in, w["part0"])  # dW_0 = dz_1^T X
         sums.append(S(w["part0"].data_ptr(), g_wg, W * Np0, Np0, W, self.d_in, grads[0].data_ptr(), self.d_in))
