@@ -86,11 +86,12 @@ __device__ __forceinline__ float lattice(const FieldAxis& a, int i, int R) {
 // such rows: where the lattice is twice as fine as the grid that is two loads
 // and four multiply-adds a point, instead of eight gathers, sixteen
 // multiply-adds and a division.
-// Bound: the 4 bytes written per point and instruction issue.  512^3 points of
-// a 256^3 grid: 771 us with a warp per lattice row and eight gathers a point,
-// 226 us with the corner values kept over the walk but all eight weighted for
-// each point, 164 us now.  (4 i and 16 rows: 8 rows 182 us, 32 rows 168 us, 2 i
-// 170 us; the next grid row loaded ahead 179 us.)
+// Bound: the 4 bytes written per point (79 us of HBM) and instruction issue.
+// 512^3 points of a 256^3 grid: 771 us with a warp per lattice row and eight
+// gathers a point, 226 us with the corner values kept over the walk but all
+// eight weighted for each point, 164 us with rows summed once, 142 us with the
+// planes' shared rows read once and the next row on its way.  (16 rows: 8 rows
+// 141 us, 32 rows 146 us.)
 constexpr int FIELD_NI = 4;
 constexpr int FIELD_ROWS = 16;
 constexpr int FIELD_THREADS = 128;
@@ -103,19 +104,17 @@ struct FieldCols {
   unsigned inside;
 };
 
-// ALL: every corner of the CTA's rows is inside.
-template <bool ALL>
 __device__ __forceinline__ void field_load(const float* __restrict__ sdf, const GridGeom& g, int jj,
                                            const FieldCols& c, float (&v)[FIELD_NI][2][2]) {
   const bool in_j = jj >= 0 && jj < g.Y;
-  const float* row = sdf + (ALL || in_j ? jj : 0) * g.Z;
+  const float* row = sdf + (in_j ? jj : 0) * g.Z;
 #pragma unroll
   for (int p = 0; p < FIELD_NI; ++p)
 #pragma unroll
     for (int di = 0; di < 2; ++di)
 #pragma unroll
       for (int dk = 0; dk < 2; ++dk)
-        v[p][di][dk] = ALL || (in_j && ((c.inside >> (4 * p + 2 * di + dk)) & 1u)) ? __ldg(row + c.col[p][di] + dk) : 0.f;
+        v[p][di][dk] = in_j && ((c.inside >> (4 * p + 2 * di + dk)) & 1u) ? __ldg(row + c.col[p][di] + dk) : 0.f;
 }
 
 __device__ __forceinline__ void field_sum(const FieldCols& c, const float (&v)[FIELD_NI][2][2],
@@ -126,15 +125,79 @@ __device__ __forceinline__ void field_sum(const FieldCols& c, const float (&v)[F
              c.wi[p][1] * (c.wk[0] * v[p][1][0] + c.wk[1] * v[p][1][1]);
 }
 
-template <bool ALL>
+// The walk for CTAs whose corners all lie inside the grid and whose FIELD_NI
+// lattice planes are at most one grid plane apart (a lattice no coarser than
+// the grid): bit p - 1 of PAT says whether plane p lies one grid plane above
+// plane p - 1.  The planes then share their rows: popcount(PAT) + 2 of them are
+// read instead of two for each of the four.
+template <int PAT>
+__device__ __forceinline__ void field_walk_in(const float* __restrict__ sdf, const GridGeom& g,
+                                              const float2* __restrict__ row_w, const int* __restrict__ row_j0,
+                                              int rows, int n_i, int64_t R, const FieldCols& c,
+                                              float* __restrict__ o) {
+  constexpr int OFF[FIELD_NI] = {0, PAT & 1, (PAT & 1) + ((PAT >> 1) & 1), (PAT & 1) + ((PAT >> 1) & 1) + (PAT >> 2)};
+  constexpr int N = OFF[FIELD_NI - 1] + 2;
+  const float* base = sdf + c.col[0][0];
+  const int plane = g.Y * g.Z;
+  float v[N][2];       // the corners of the grid row after hi's, on their way
+  auto load = [&](int jj) {
+    const float* row = base + min(jj, g.Y - 1) * g.Z;
+#pragma unroll
+    for (int q = 0; q < N; ++q) {
+      v[q][0] = __ldg(row + q * plane);
+      v[q][1] = __ldg(row + q * plane + 1);
+    }
+  };
+  auto sums = [&](float (&sum)[FIELD_NI]) {
+    float zl[N];
+#pragma unroll
+    for (int q = 0; q < N; ++q) zl[q] = c.wk[0] * v[q][0] + c.wk[1] * v[q][1];
+#pragma unroll
+    for (int p = 0; p < FIELD_NI; ++p) sum[p] = c.wi[p][0] * zl[OFF[p]] + c.wi[p][1] * zl[OFF[p] + 1];
+  };
+  float lo[FIELD_NI], hi[FIELD_NI];
+  float* dst[FIELD_NI];
+#pragma unroll
+  for (int p = 0; p < FIELD_NI; ++p) dst[p] = o + p * R * R;
+  int at = row_j0[0];
+  load(at);
+  sums(lo);
+  load(at + 1);
+  sums(hi);
+  load(at + 2);
+  for (int r = 0; r < rows; ++r) {
+    const int j0 = row_j0[r];
+    if (j0 != at) {
+      if (j0 == at + 1) {
+#pragma unroll
+        for (int p = 0; p < FIELD_NI; ++p) lo[p] = hi[p];
+      } else {
+        load(j0);
+        sums(lo);
+        load(j0 + 1);
+      }
+      sums(hi);
+      at = j0;
+      load(at + 2);
+    }
+    const float2 wj = row_w[r];
+#pragma unroll
+    for (int p = 0; p < FIELD_NI; ++p) {
+      if (p < n_i) __stcs(dst[p], wj.x * lo[p] + wj.y * hi[p]);
+      dst[p] += R;
+    }
+  }
+}
+
+// Any lattice: every corner is checked against the grid.
 __device__ __forceinline__ void field_walk(const float* __restrict__ sdf, const GridGeom& g,
                                            const float2* __restrict__ row_w, const int* __restrict__ row_j0, int rows,
                                            int n_i, int64_t R, const FieldCols& c, float* __restrict__ o) {
   float lo[FIELD_NI], hi[FIELD_NI], v[FIELD_NI][2][2];
   int at = row_j0[0];
-  field_load<ALL>(sdf, g, at, c, v);
+  field_load(sdf, g, at, c, v);
   field_sum(c, v, lo);
-  field_load<ALL>(sdf, g, at + 1, c, v);
+  field_load(sdf, g, at + 1, c, v);
   field_sum(c, v, hi);
   for (int r = 0; r < rows; ++r, o += R) {
     const int j0 = row_j0[r];
@@ -143,10 +206,10 @@ __device__ __forceinline__ void field_walk(const float* __restrict__ sdf, const 
 #pragma unroll
         for (int p = 0; p < FIELD_NI; ++p) lo[p] = hi[p];
       } else {
-        field_load<ALL>(sdf, g, j0, c, v);
+        field_load(sdf, g, j0, c, v);
         field_sum(c, v, lo);
       }
-      field_load<ALL>(sdf, g, j0 + 1, c, v);
+      field_load(sdf, g, j0 + 1, c, v);
       field_sum(c, v, hi);
       at = j0;
     }
@@ -162,6 +225,8 @@ __global__ void __launch_bounds__(FIELD_THREADS) sdf_field_kernel(const float* _
                                                                   float sign, float* __restrict__ out) {
   __shared__ float2 row_w[FIELD_ROWS];   // the rows' two y weights, times sign
   __shared__ int row_j0[FIELD_ROWS];
+  __shared__ float plane_t[FIELD_NI];
+  __shared__ int plane_i0[FIELD_NI];
   const int ib = blockIdx.z * FIELD_NI, jb = blockIdx.y * FIELD_ROWS;
   const int rows = min(FIELD_ROWS, R - jb), n_i = min(FIELD_NI, R - ib);
   bool rows_in = true;
@@ -172,6 +237,12 @@ __global__ void __launch_bounds__(FIELD_THREADS) sdf_field_kernel(const float* _
     row_w[threadIdx.x] = make_float2(sign * (1.f - tj), sign * tj);
     row_j0[threadIdx.x] = j0;
     rows_in = j0 >= 0 && j0 < g.Y - 1;
+  } else if ((int)threadIdx.x >= 32 && (int)threadIdx.x < 32 + FIELD_NI) {
+    const int p = (int)threadIdx.x - 32;
+    const float fi = world_to_index(g, 0, lattice(ax, min(ib + p, R - 1), R)), fi0 = floorf(fi);
+    plane_i0[p] = (int)fi0;
+    plane_t[p] = fi - fi0;
+    rows_in = plane_i0[p] >= 0 && plane_i0[p] < g.X - 1;
   }
   rows_in = __syncthreads_and(rows_in);
   const int k = blockIdx.x * FIELD_THREADS + threadIdx.x;
@@ -183,13 +254,16 @@ __global__ void __launch_bounds__(FIELD_THREADS) sdf_field_kernel(const float* _
   c.wk[0] = 1.f - tk;
   c.wk[1] = tk;
   c.inside = 0;
+  int pat = 0;         // -1: planes further apart
 #pragma unroll
   for (int p = 0; p < FIELD_NI; ++p) {
-    const float fi = world_to_index(g, 0, lattice(ax, min(ib + p, R - 1), R)), fi0 = floorf(fi);
-    const int i0 = (int)fi0;
-    const float ti = fi - fi0;
-    c.wi[p][0] = 1.f - ti;
-    c.wi[p][1] = ti;
+    const int i0 = plane_i0[p];
+    c.wi[p][0] = 1.f - plane_t[p];
+    c.wi[p][1] = plane_t[p];
+    if (p > 0) {
+      const int step = i0 - plane_i0[p - 1];
+      pat = step < 0 || step > 1 || pat < 0 ? -1 : pat | step << (p - 1);
+    }
 #pragma unroll
     for (int di = 0; di < 2; ++di) {
       const int ii = i0 + di;
@@ -201,11 +275,19 @@ __global__ void __launch_bounds__(FIELD_THREADS) sdf_field_kernel(const float* _
     }
   }
   float* o = out + ((int64_t)ib * R + jb) * R + k;
-  const unsigned all = (1u << (4 * FIELD_NI)) - 1u;
-  if (rows_in && c.inside == all)
-    field_walk<true>(sdf, g, row_w, row_j0, rows, n_i, R, c, o);
-  else
-    field_walk<false>(sdf, g, row_w, row_j0, rows, n_i, R, c, o);
+  if (rows_in && pat >= 0 && k0 >= 0 && k0 < g.Z - 1) {
+    switch (pat) {
+      case 0: return field_walk_in<0>(sdf, g, row_w, row_j0, rows, n_i, R, c, o);
+      case 1: return field_walk_in<1>(sdf, g, row_w, row_j0, rows, n_i, R, c, o);
+      case 2: return field_walk_in<2>(sdf, g, row_w, row_j0, rows, n_i, R, c, o);
+      case 3: return field_walk_in<3>(sdf, g, row_w, row_j0, rows, n_i, R, c, o);
+      case 4: return field_walk_in<4>(sdf, g, row_w, row_j0, rows, n_i, R, c, o);
+      case 5: return field_walk_in<5>(sdf, g, row_w, row_j0, rows, n_i, R, c, o);
+      case 6: return field_walk_in<6>(sdf, g, row_w, row_j0, rows, n_i, R, c, o);
+      default: return field_walk_in<7>(sdf, g, row_w, row_j0, rows, n_i, R, c, o);
+    }
+  }
+  field_walk(sdf, g, row_w, row_j0, rows, n_i, R, c, o);
 }
 
 static FieldAxis field_axis(float start, float end, int64_t R) {
