@@ -1135,6 +1135,22 @@ typedef struct {
 } vx_womask_composite_args;
 int vx_womask_composite(const vx_womask_composite_args* args, void* stream);
 
+/* ---- photometric loss (run.py:604-627) -------------------------------------
+ * loss = w_main mse(rgb, target) + w_entropy H(p) + w_rgb0 mse(rgb0, target),
+ * p = clamp(*alphainv_last, 1e-6, 1 - 1e-6), H the binary entropy; rgb0 and
+ * alphainv_last may be null (no such term).  n = elements of each colour
+ * tensor; scratch: vx_photo_loss_scratch_bytes(n) bytes (0 up to 65536
+ * elements), 16-byte aligned. */
+size_t vx_photo_loss_scratch_bytes(int64_t n);
+int vx_photo_loss(const float* rgb, const float* rgb0, const float* target, int64_t n, const float* alphainv_last,
+                  float w_main, float w_rgb0, float w_entropy, float* loss, void* scratch, size_t scratch_bytes,
+                  void* stream);
+/* Gradients for the upstream scalar *g; d_alphainv [n_alphainv] is zero but for
+ * its last element. */
+int vx_photo_loss_backward(const float* rgb, const float* rgb0, const float* target, int64_t n,
+                           const float* alphainv_last, float w_main, float w_rgb0, float w_entropy, const float* g,
+                           float* d_rgb, float* d_rgb0, float* d_alphainv, int64_t n_alphainv, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -70,12 +70,17 @@ _SIGNATURES = {
                                      c_ptr],
     "vx_grid_clear_touched": [c_ptr, c_ptr, c_i64, c_i64, c_ptr],
     "vx_cumdist_thres": [c_ptr, c_i64, c_i64, c_f32, c_ptr, c_ptr],
+    "vx_photo_loss_scratch_bytes": [c_i64],
+    "vx_photo_loss": [c_ptr, c_ptr, c_ptr, c_i64, c_ptr, c_f32, c_f32, c_f32, c_ptr, c_ptr, c_size, c_ptr],
+    "vx_photo_loss_backward": [c_ptr, c_ptr, c_ptr, c_i64, c_ptr, c_f32, c_f32, c_f32, c_ptr, c_ptr, c_ptr, c_ptr,
+                               c_i64, c_ptr],
 }
 
 _RESTYPES = {
     "vx_status_string": C.c_char_p,
     "vx_cuda_error_string": C.c_char_p,
     "vx_scan_scratch_bytes": c_size,
+    "vx_photo_loss_scratch_bytes": c_size,
     "vx_launch_count": C.c_ulonglong,
 }
 

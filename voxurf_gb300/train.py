@@ -12,19 +12,90 @@ from __future__ import annotations
 import torch
 import torch.nn.functional as F
 
+from . import _native
+from ._torch import call, ptr, scratch, stream_ptr
 from .utils import Adam
+
+
+class _PhotoLoss(torch.autograd.Function):
+    """fine_loss in one launch forward and one backward (vx_photo_loss) on
+    contiguous FP32 CUDA tensors.  rgb0 / alphainv may be None."""
+
+    @staticmethod
+    def forward(ctx, rgb, rgb0, alphainv, target, w_main, w_rgb0, w_entropy):
+        n = rgb.numel()
+        nb = int(_native.load().vx_photo_loss_scratch_bytes(n))
+        tmp = scratch(nb, rgb.device) if nb else None
+        loss = torch.empty((), dtype=torch.float32, device=rgb.device)
+        call("vx_photo_loss", ptr(rgb), ptr(rgb0), ptr(target), n, _last_ptr(alphainv), w_main, w_rgb0, w_entropy,
+             ptr(loss), ptr(tmp), nb, stream_ptr(rgb.device))
+        ctx.save_for_backward(rgb, rgb0, alphainv, target)
+        ctx.weights = (w_main, w_rgb0, w_entropy)
+        return loss
+
+    @staticmethod
+    def backward(ctx, g):
+        rgb, rgb0, alphainv, target = ctx.saved_tensors
+        w_main, w_rgb0, w_entropy = ctx.weights
+        if torch.is_grad_enabled():
+            # create_graph: the same gradients from differentiable operations
+            norm = 2.0 / rgb.numel()
+            d_rgb = norm * (rgb - target) * (g * w_main)
+            d_rgb0 = None if rgb0 is None else norm * (rgb0 - target) * (g * w_rgb0)
+            d_a = None
+            if alphainv is not None:
+                x = alphainv[-1]
+                p = x.clamp(1e-6, 1 - 1e-6)
+                d = torch.where((x >= 1e-6) & (x <= 1 - 1e-6), torch.log(1 - p) - torch.log(p), torch.zeros_like(p))
+                d_a = F.pad((g * w_entropy * d)[None], (alphainv.numel() - 1, 0))
+            return d_rgb, d_rgb0, d_a, None, None, None, None
+        g = g.contiguous()
+        d_rgb = torch.empty_like(rgb)
+        d_rgb0 = None if rgb0 is None else torch.empty_like(rgb0)
+        d_a = None if alphainv is None else torch.empty_like(alphainv)
+        call("vx_photo_loss_backward", ptr(rgb), ptr(rgb0), ptr(target), rgb.numel(), _last_ptr(alphainv), w_main,
+             w_rgb0, w_entropy, ptr(g), ptr(d_rgb), ptr(d_rgb0), ptr(d_a), 0 if d_a is None else d_a.numel(),
+             stream_ptr(rgb.device))
+        return d_rgb, d_rgb0, d_a, None, None, None, None
+
+
+def _last_ptr(t):
+    return None if t is None else t.data_ptr() + 4 * (t.numel() - 1)
+
+
+def _plain(t) -> bool:
+    return type(t) is torch.Tensor and t.is_cuda and t.dtype == torch.float32 and t.is_contiguous() and t.numel() > 0
+
+
+def _one_launch(rgb, rgb0, alphainv, target, weights) -> bool:
+    """Whether the loss kernels may stand for the chain of torch operations:
+    plain tensors of one shape on one device, a target without a gradient, plain
+    weights, and no transform, forward-mode, tracing or compiling around."""
+    ts = [t for t in (rgb, rgb0, target) if t is not None]
+    return (all(_plain(t) and t.shape == rgb.shape and t.device == rgb.device for t in ts)
+            and (alphainv is None or (_plain(alphainv) and alphainv.dim() == 1 and alphainv.device == rgb.device))
+            and rgb.device.index == torch.cuda.current_device() and not target.requires_grad
+            and all(type(w) in (int, float) for w in weights)
+            and torch.autograd.forward_ad._current_level < 0 and not torch._C._are_functorch_transforms_active()
+            and not torch.jit.is_tracing() and not torch.compiler.is_compiling())
 
 
 def fine_loss(ret, target, weight_main=1.0, weight_entropy_last=0.001, weight_rgb0=0.5):
     """run.py:604-636 with the fine dtu_e2e weights (configs/dtu_e2e/fine.py:104-105
     and the surf_train default weight_entropy_last, default_fine_s.py:63)."""
-    loss = weight_main * F.mse_loss(ret["rgb_marched"], target)
-    if weight_entropy_last > 0:
+    rgb = ret["rgb_marched"]
+    alphainv = ret["alphainv_cum"] if weight_entropy_last > 0 else None
+    rgb0 = ret["rgb_marched0"] if weight_rgb0 > 0 and "rgb_marched0" in ret else None
+    if _one_launch(rgb, rgb0, alphainv, target, (weight_main, weight_entropy_last, weight_rgb0)):
+        return _PhotoLoss.apply(rgb, rgb0, alphainv, target, float(weight_main), float(weight_rgb0),
+                                float(weight_entropy_last))
+    loss = weight_main * F.mse_loss(rgb, target)
+    if alphainv is not None:
         # run.py:608: [..., -1] of the 1-D alphainv_cum selects the last ray
-        pout = ret["alphainv_cum"][..., -1].clamp(1e-6, 1 - 1e-6)
+        pout = alphainv[..., -1].clamp(1e-6, 1 - 1e-6)
         loss = loss + weight_entropy_last * (-(pout * torch.log(pout) + (1 - pout) * torch.log(1 - pout)).mean())
-    if weight_rgb0 > 0 and "rgb_marched0" in ret:
-        loss = loss + F.mse_loss(ret["rgb_marched0"], target) * weight_rgb0
+    if rgb0 is not None:
+        loss = loss + F.mse_loss(rgb0, target) * weight_rgb0
     return loss
 
 
