@@ -4,9 +4,11 @@
 // As separate elementwise and reduction launches the loss of an 8192-ray batch
 // was about 50 launches of 1-5 us, over a millisecond of host time in which the
 // GPU waited; here it is one launch forward and one backward: the FP32 training
-// step 3,145 -> 2,491 us.  Bound: launch latency (three tensors of 98 KB).  The squared errors are summed in 64 bits
-// in a fixed order; the gradients are formed as the elementwise chain forms
-// them (the norm 2/n times the difference, times the upstream scalar).
+// step 3,145 -> 2,368 us.  Bound: latency (three tensors of 98 KB).  A thread
+// sums its squares (at most 64) in FP32 and the threads' sums are added in 64
+// bits, in a fixed order: with every addition in 64 bits the one block took 33
+// us, 10 us now.  The gradients are formed as the elementwise chain forms them
+// (the norm 2/n times the difference, times the upstream scalar).
 #include <algorithm>
 
 #include "common.cuh"
@@ -54,19 +56,18 @@ __device__ __forceinline__ float photo_value(const PhotoLoss& P, double s, doubl
 __global__ void __launch_bounds__(PL_THREADS) photo_loss_kernel(PhotoLoss P, double2* __restrict__ part,
                                                                float* __restrict__ loss) {
   __shared__ double warps[PL_THREADS / 32];
-  double s = 0.0, s0 = 0.0;
+  float sf = 0.f, s0f = 0.f;
   const int64_t end = min(P.n, (int64_t)(blockIdx.x + 1) * PL_PER_BLOCK);
-#pragma unroll 4
+#pragma unroll 8
   for (int64_t i = (int64_t)blockIdx.x * PL_PER_BLOCK + threadIdx.x; i < end; i += PL_THREADS) {
     const float t = P.target[i], d = fsub(P.rgb[i], t);
-    s += (double)fmul(d, d);
+    sf = fadd(sf, fmul(d, d));
     if (P.rgb0) {
       const float d0 = fsub(P.rgb0[i], t);
-      s0 += (double)fmul(d0, d0);
+      s0f = fadd(s0f, fmul(d0, d0));
     }
   }
-  s = block_sum(s, warps);
-  s0 = block_sum(s0, warps);
+  const double s = block_sum((double)sf, warps), s0 = block_sum((double)s0f, warps);
   if (threadIdx.x == 0) {
     if (gridDim.x == 1) *loss = photo_value(P, s, s0);
     else part[blockIdx.x] = make_double2(s, s0);
