@@ -28,11 +28,15 @@
 //                         at a time while the previous 64 are multiplied;
 //   split_wgrad_kernel    D = A^T B over a CTA's rows (dz^T h): both operands
 //                         split into MN-major shared-memory tiles of 32 rows.
+//                         A warp of its own issues the MMAs (24 of them take a
+//                         thread ~2,000 cycles: a warp that also splits kept
+//                         the others waiting, 105 -> 91 us), and the partials
+//                         leave in whole sectors (4 us).
 // 131,003 rows, 192 x 192: the row GEMM with mask and column sums 176 -> 84 us
-// (its three FP32 matrices take 44 us of HBM), the weight gradient 208 -> 105
+// (its three FP32 matrices take 44 us of HBM), the weight gradient 208 -> 87
 // us (30 us of HBM).  Bound now: the row GEMM's loads and stores beside its
-// MMAs; in the weight gradient the splitting and its barrier per 32 rows (with
-// a sixth of the MMAs it still takes 85 us, without the loads 88 us).
+// MMAs; in the weight gradient the MMAs and the splitting of 32 rows, each
+// about 1 us, two stages deep, and about 10 us of filling and storing per CTA.
 #include <algorithm>
 
 #include "mlp_f32.cuh"
@@ -393,6 +397,13 @@ int split_rowgemm_launch(const RowGemmParams& P, cudaStream_t st) {
   return P.Np == 80 ? rowgemm_go<128, 80>(P, st) : rowgemm_go<128, 64>(P, st);
 }
 
+// A whole 32-byte sector in one store: two of 16 bytes would each write half.
+__device__ __forceinline__ void st_sector(float* p, const float* v) {
+  asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]),
+               "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
+               : "memory");
+}
+
 // ============================================================================
 // D = A^T B over a CTA's rows
 // ============================================================================
@@ -410,10 +421,11 @@ struct WgradGeo {
   static constexpr int TM_COLS = COLS <= 128 ? 128 : (COLS <= 256 ? 256 : 512);
   static constexpr int A_PART = WS_ROWS * M * 2, B_PART = WS_ROWS * NC * 2;   // bytes of one part
   static constexpr int SLOT = 3 * (A_PART + B_PART);
-  // 12 or 8 warps: TMEM lane quarter = warp % 4, column part = warp / 4.  16
-  // threads (8 rows x 2 float4s) take a core matrix, the M / 8 groups of
-  // threads a row block of A per item; the items of B follow.
-  static constexpr int THREADS = 2 * M, TG = THREADS / 16, PARTS = THREADS / 128;
+  // 12 or 8 warps split: TMEM lane quarter = warp % 4, column part = warp / 4.
+  // 16 threads (8 rows x 2 float4s) take a core matrix, the M / 8 groups of
+  // threads a row block of A per item; the items of B follow.  One more warp
+  // issues the MMAs.
+  static constexpr int THREADS = 2 * M, TG = THREADS / 16, PARTS = THREADS / 128, WARPS = THREADS / 32;
   static constexpr int A_ITEMS = WS_ROWS / 8, B_ITEMS = (WS_ROWS / 8 * (NC / 8) + TG - 1) / TG;
   static constexpr int ITEMS = A_ITEMS + B_ITEMS;
   static constexpr int BLOCKS = (NC / 16 + PARTS - 1) / PARTS;     // 16-column blocks of D per warp, every PARTS-th
@@ -423,12 +435,13 @@ struct WgradGeo {
 };
 
 template <int M, int NC>
-__global__ void __launch_bounds__(WgradGeo<M, NC>::THREADS, 1) split_wgrad_kernel(WgradParams P, int NP, int n_ranges, int* err) {
+__global__ void __launch_bounds__(WgradGeo<M, NC>::THREADS + 32, 1) split_wgrad_kernel(WgradParams P, int NP, int n_ranges, int* err) {
   using G = WgradGeo<M, NC>;
   extern __shared__ __align__(1024) uint8_t smem[];
   float4* raw = reinterpret_cast<float4*>(smem + (size_t)WS_SLOTS * G::SLOT);   // [WS_RAW][ITEMS][G::THREADS]
   uint64_t* bar = reinterpret_cast<uint64_t*>(smem + (size_t)WS_SLOTS * G::SLOT + (size_t)WS_RAW * G::RAW);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar + WS_SLOTS);
+  uint64_t* full = bar + WS_SLOTS;       // a slot's parts are written; bar: its MMAs have run
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(full + WS_SLOTS);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int quarter = warp & 3, part = warp >> 2;
   // the column halves of a row range are neighbours: the second reads A from L2
@@ -441,7 +454,10 @@ __global__ void __launch_bounds__(WgradGeo<M, NC>::THREADS, 1) split_wgrad_kerne
 
   if (warp == 0) alloc(tmem_slot, G::TM_COLS);
   if (tid == 0) {
-    for (int s = 0; s < WS_SLOTS; ++s) mbar_init(bar + s, 1);
+    for (int s = 0; s < WS_SLOTS; ++s) {
+      mbar_init(bar + s, 1);
+      mbar_init(full + s, G::WARPS);
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   fence_before();
@@ -522,68 +538,76 @@ __global__ void __launch_bounds__(WgradGeo<M, NC>::THREADS, 1) split_wgrad_kerne
     }
   };
 
+  if (warp < G::WARPS) {
 #pragma unroll
-  for (int st = 0; st < WS_RAW; ++st) {
-    if (st < nst) load(st);
-    cp_async_commit();
-  }
-  for (int st = 0; st < nst; ++st) {
-    const int slot = st % WS_SLOTS;
-    if (st >= WS_SLOTS) ok = mbar_wait(bar + slot, (uint32_t)((st / WS_SLOTS - 1) & 1)) && ok;
-    asm volatile("cp.async.wait_group %0;" ::"n"(WS_RAW - 1) : "memory");
-    uint8_t* base = smem + (size_t)slot * G::SLOT;
-    const float4* mine = raw + (size_t)(st % WS_RAW) * (G::ITEMS * G::THREADS) + tid;
-#pragma unroll
-    for (int q = 0; q < G::A_ITEMS; ++q) put(base + a_dst + q * (M * 16), G::A_PART, mine[q * G::THREADS], bad);
-#pragma unroll
-    for (int q = 0; q < G::B_ITEMS; ++q)
-      if (b_row[q] >= 0)
-        put(base + 3 * G::A_PART + b_dst[q], G::B_PART, mine[(G::A_ITEMS + q) * G::THREADS], bad);
-    if (st + WS_RAW < nst) load(st + WS_RAW);
-    cp_async_commit();
-    const bool first = st % WS_GROUP == 0;
-    if (first && st > 0) drain(st - 1);
-    fence_async_smem();
-    fence_before();
-    if (__syncthreads_or(!ok)) {
-      ok = false;
-      break;
+    for (int st = 0; st < WS_RAW; ++st) {
+      if (st < nst) load(st);
+      cp_async_commit();
     }
-    if (tid == 0) {
+    for (int st = 0; st < nst && ok; ++st) {
+      const int slot = st % WS_SLOTS;
+      if (st >= WS_SLOTS) ok = mbar_wait(bar + slot, (uint32_t)((st / WS_SLOTS - 1) & 1)) && ok;
+      asm volatile("cp.async.wait_group %0;" ::"n"(WS_RAW - 1) : "memory");
+      uint8_t* base = smem + (size_t)slot * G::SLOT;
+      const float4* mine = raw + (size_t)(st % WS_RAW) * (G::ITEMS * G::THREADS) + tid;
+#pragma unroll
+      for (int q = 0; q < G::A_ITEMS; ++q) put(base + a_dst + q * (M * 16), G::A_PART, mine[q * G::THREADS], bad);
+#pragma unroll
+      for (int q = 0; q < G::B_ITEMS; ++q)
+        if (b_row[q] >= 0)
+          put(base + 3 * G::A_PART + b_dst[q], G::B_PART, mine[(G::A_ITEMS + q) * G::THREADS], bad);
+      if (st + WS_RAW < nst) load(st + WS_RAW);
+      cp_async_commit();
+      if (st > 0 && st % WS_GROUP == 0) drain(st - 1);
+      fence_async_smem();
+      fence_before();
+      ok = __all_sync(0xffffffffu, ok);
+      if (lane == 0) mbar_arrive(full + slot);
+    }
+    cp_async_wait_all();
+    if (nst > 0 && ok) drain(nst - 1);
+  } else {
+    const uint32_t id = idesc(TILE_M, NC, 1, 1);
+    const int pa[6] = {0, 2, 1, 0, 1, 0}, pb[6] = {2, 0, 1, 1, 0, 0};   // the small products first
+    for (int st = 0; st < nst && ok; ++st) {
+      const int slot = st % WS_SLOTS;
+      ok = __all_sync(0xffffffffu, mbar_wait(full + slot, (uint32_t)((st / WS_SLOTS) & 1)));
       fence_after();
-      const uint32_t a_s = smem_u32(base), b_s = a_s + 3 * G::A_PART;
-      const uint32_t id = idesc(TILE_M, NC, 1, 1);
-      const int pa[6] = {0, 2, 1, 0, 1, 0}, pb[6] = {2, 0, 1, 1, 0, 0};   // the small products first
-      for (int mt = 0; mt < G::MT; ++mt)
+      if (lane == 0 && ok) {
+        const uint32_t a_s = smem_u32(smem + (size_t)slot * G::SLOT);
+        // (a descriptor's address field holds 16-byte units and does not carry)
+        const uint64_t a_d = desc(a_s, M * 16, 128), b_d = desc(a_s + 3 * G::A_PART, NC * 16, 128);
+        const bool first = st % WS_GROUP == 0;
 #pragma unroll
-        for (int q = 0; q < 6; ++q) {
-          const bool hh = q == 5;
-          const uint32_t d = tmem + (uint32_t)((hh ? G::D_HI : 0) + mt * NC);
+        for (int mt = 0; mt < G::MT; ++mt)
 #pragma unroll
-          for (int ks = 0; ks < WS_ROWS / 16; ++ks) {
-            const uint64_t ad = desc(a_s + (uint32_t)(pa[q] * G::A_PART + 2 * ks * (M * 16) + mt * 16 * 128), M * 16, 128);
-            const uint64_t bd = desc(b_s + (uint32_t)(pb[q] * G::B_PART + 2 * ks * (NC * 16)), NC * 16, 128);
-            mma_ss(d, ad, bd, id, !first || ks > 0 || (!hh && q > 0));
+          for (int q = 0; q < 6; ++q) {
+            const bool hh = q == 5;
+            const uint32_t d = tmem + (uint32_t)((hh ? G::D_HI : 0) + mt * NC);
+#pragma unroll
+            for (int ks = 0; ks < WS_ROWS / 16; ++ks)
+              mma_ss(d, a_d + (uint64_t)((pa[q] * G::A_PART + 2 * ks * (M * 16) + mt * 16 * 128) / 16),
+                     b_d + (uint64_t)((pb[q] * G::B_PART + 2 * ks * (NC * 16)) / 16), id,
+                     !first || ks > 0 || (!hh && q > 0));
           }
-        }
-      commit(bar + slot);
+        commit(bar + slot);
+      }
+      __syncwarp();
     }
   }
-  cp_async_wait_all();
-  if (nst > 0 && ok) drain(nst - 1);
   if (!ok) set_device_error(err, VX_ERR_TIMEOUT);
   float* out = P.part + (size_t)range * M * NP;
   if (__syncthreads_or(bad)) {
     // a value without parts among the CTA's rows: plain FP32 sums, in the
     // order of the CUDA-core kernel
-    for (int i = tid; i < M * NC; i += G::THREADS) {
+    for (int i = tid; i < M * NC; i += G::THREADS + 32) {
       const int m = i / NC, n = n0 + i % NC;
       float v = 0.f;
       if (n < P.N)
         for (int64_t r = r0; r < r1; ++r) v = fmaf(P.A[r * P.lda + m], P.B[r * P.ldb + n], v);
       out[(size_t)m * NP + n] = v;
     }
-  } else {
+  } else if (warp < G::WARPS) {
 #pragma unroll
     for (int mt = 0; mt < G::MT; ++mt) {
       const int m = mt * TILE_M + 32 * quarter + lane;
@@ -593,9 +617,7 @@ __global__ void __launch_bounds__(WgradGeo<M, NC>::THREADS, 1) split_wgrad_kerne
         const int c = 16 * (G::PARTS * b + part);
         if (c >= NC) break;
 #pragma unroll
-        for (int e = 0; e < 16; e += 4)
-          *reinterpret_cast<float4*>(out + (size_t)m * NP + n0 + c + e) =
-              make_float4(acc[mt][b][e], acc[mt][b][e + 1], acc[mt][b][e + 2], acc[mt][b][e + 3]);
+        for (int e = 0; e < 16; e += 8) st_sector(out + (size_t)m * NP + n0 + c + e, acc[mt][b] + e);
       }
     }
   }
@@ -611,7 +633,7 @@ bool split_wgrad_takes(const WgradParams& P, int MP, int NP) {
   const uintptr_t a16 = reinterpret_cast<uintptr_t>(P.A) | reinterpret_cast<uintptr_t>(P.B) |
                         reinterpret_cast<uintptr_t>(P.part);
   return (MP == 128 || MP == 192) && P.M == MP && (NP == MP || NP == 80 || NP == 64) && P.lda % 4 == 0 &&
-         P.ldb % 4 == 0 && a16 % 16 == 0;
+         P.ldb % 4 == 0 && a16 % 16 == 0 && reinterpret_cast<uintptr_t>(P.part) % 32 == 0;
 }
 
 template <int M, int NC>
@@ -620,7 +642,7 @@ static int wgrad_go(const WgradParams& P, int NP, unsigned grid, cudaStream_t st
   const cudaError_t e =
       cudaFuncSetAttribute(split_wgrad_kernel<M, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::SMEM);
   if (e != cudaSuccess) return cuda_status(e);
-  split_wgrad_kernel<M, NC><<<grid * (unsigned)(NP / NC), G::THREADS, G::SMEM, st>>>(P, NP, (int)grid,
+  split_wgrad_kernel<M, NC><<<grid * (unsigned)(NP / NC), G::THREADS + 32, G::SMEM, st>>>(P, NP, (int)grid,
                                                                                    device_error_ptr());
   return launch_status();
 }
