@@ -787,9 +787,11 @@ typedef struct {
 /* Up to 8 jobs in one launch. */
 int vx_mlp_train_reduce(const vx_mlp_reduce_job* jobs, int n_jobs, void* stream);
 
-/* ---- colour-MLP training in plain FP32 on the CUDA cores (the same layers
- *      as above with FP32 operands and FP32 fused multiply-adds; the output
- *      layer runs in vx_mlp_head / vx_mlp_head_backward).  Weights enter as
+/* ---- colour-MLP training in plain FP32 (the same layers as above with FP32
+ *      operands: fused multiply-adds on the CUDA cores, and for the backward
+ *      GEMMs of widths 128 and 192 with aligned buffers the tensor cores on
+ *      operands split into three BF16 parts, no less exact; the output layer
+ *      runs in vx_mlp_head / vx_mlp_head_backward).  Weights enter as
  *      Bt [Kp][Np] FP32 (vx_mlp_train_pack mode 3), Np in {32, 64, 80, 128,
  *      192}. ---- */
 typedef struct {

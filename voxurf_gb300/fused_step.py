@@ -26,7 +26,7 @@ is captured, and is replayed; re-running part B is idempotent because it
 clears its accumulators first.
 
 The colour MLPs run on the engines of mlp.py (the tcgen05 kernels for BF16
-rows, the FP32 CUDA-core kernels for FP32 rows); their input rows are padded
+rows, the FP32 kernels for FP32 rows); their input rows are padded
 to the engine's row stride, and the rgbnet forward writes its logits straight
 into the k-branch rows (k_res).
 """

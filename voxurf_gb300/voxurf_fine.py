@@ -16,7 +16,7 @@ the fused sm_103a kernels of libvoxurf_gb300.so:
       and k0, then the smoothing adjoint.
   rgbnet / k_rgbnet: nn.Linear stacks run by the library's own MLP
       engines (mlp.apply_mlp): tcgen05 BF16 kernels in the mixed-precision
-      mode, CUDA-core FP32 kernels in the plain mode.
+      mode, FP32 kernels in the plain mode.
   _FineComposite (autograd.Function): per-ray compositing and its backward.
 
 precision='fp32' is the plain FP32 path; precision='bf16' samples k0 from a
