@@ -143,3 +143,22 @@ def test_wgrad_values_without_parts(cuda, where, value):
     cols = slice(96, 192) if where == "B" else slice(None)
     assert torch.equal(split[i][:, cols].view(torch.int32), plain[i][:, cols].view(torch.int32))
     torch.testing.assert_close(split, plain, rtol=1e-4, atol=1e-4, equal_nan=True)
+
+
+@pytest.mark.parametrize("offset", [0, 4, 8])
+def test_wgrad_partials_within_a_buffer(cuda, offset):
+    """Partials that start 16 but not 32 bytes into a sector are summed on the
+    CUDA cores (the tensor-core kernel stores whole sectors): exact either way,
+    and nothing beside them is written."""
+    rows, W = 1000, 192
+    g = torch.Generator().manual_seed(offset)
+    A, B = (torch.randint(-3, 4, (rows, W), generator=g).float().to(cuda) for _ in range(2))
+    grid = int(_native.load().vx_mlp_f32_wgrad_grid(rows))
+    buf = torch.full((offset + grid * W * W + 8,), 7.0, device=cuda)
+    part = buf[offset:offset + grid * W * W]
+    a = _abi.MlpF32WgradArgs()
+    a.A, a.lda, a.B, a.ldb, a.M, a.N, a.rows = ptr(A), W, ptr(B), W, W, W, rows
+    a.part, a.part_cap = part.data_ptr(), part.numel()
+    _abi.call_struct("vx_mlp_f32_wgrad", a, stream_ptr(cuda))
+    assert torch.equal(part.view(grid, W, W).double().sum(0), A.double().t() @ B.double())
+    assert (buf[:offset] == 7).all() and (buf[-8:] == 7).all()
