@@ -11,6 +11,8 @@ from __future__ import annotations
 
 import torch
 import torch.nn.functional as F
+from torch.overrides import _get_current_function_mode_stack
+from torch.utils._device import DeviceContext
 
 from . import _native
 from ._torch import call, ptr, scratch, stream_ptr
@@ -37,8 +39,9 @@ class _PhotoLoss(torch.autograd.Function):
     def backward(ctx, g):
         rgb, rgb0, alphainv, target = ctx.saved_tensors
         w_main, w_rgb0, w_entropy = ctx.weights
-        if torch.is_grad_enabled():
-            # create_graph: the same gradients from differentiable operations
+        if torch.is_grad_enabled() or _watched():
+            # create_graph, or a tracer over the backward: the same gradients
+            # from torch operations
             norm = 2.0 / rgb.numel()
             d_rgb = norm * (rgb - target) * (g * w_main)
             d_rgb0 = None if rgb0 is None else norm * (rgb0 - target) * (g * w_rgb0)
@@ -64,20 +67,30 @@ def _last_ptr(t):
 
 
 def _plain(t) -> bool:
-    return type(t) is torch.Tensor and t.is_cuda and t.dtype == torch.float32 and t.is_contiguous() and t.numel() > 0
+    return (type(t) is torch.Tensor and t.is_cuda and t.dtype == torch.float32 and t.is_contiguous() and t.numel() > 0
+            and not t.is_neg())
+
+
+def _watched() -> bool:
+    """Whether something around sees every torch operation, a proxy tracer or a
+    user's dispatch mode: it would not see the kernels.  (A default device is
+    the one function mode that only concerns factory calls.)"""
+    return torch._C._len_torch_dispatch_stack() > 0 or (
+        torch._C._len_torch_function_stack() > 0
+        and any(type(m) is not DeviceContext for m in _get_current_function_mode_stack()))
 
 
 def _one_launch(rgb, rgb0, alphainv, target, weights) -> bool:
     """Whether the loss kernels may stand for the chain of torch operations:
     plain tensors of one shape on one device, a target without a gradient, plain
-    weights, and no transform, forward-mode, tracing or compiling around."""
+    weights, and no transform, forward-mode, mode, tracing or compiling around."""
     ts = [t for t in (rgb, rgb0, target) if t is not None]
     return (all(_plain(t) and t.shape == rgb.shape and t.device == rgb.device for t in ts)
             and (alphainv is None or (_plain(alphainv) and alphainv.dim() == 1 and alphainv.device == rgb.device))
             and rgb.device.index == torch.cuda.current_device() and not target.requires_grad
             and all(type(w) in (int, float) for w in weights)
             and torch.autograd.forward_ad._current_level < 0 and not torch._C._are_functorch_transforms_active()
-            and not torch.jit.is_tracing() and not torch.compiler.is_compiling())
+            and not torch.jit.is_tracing() and not torch.compiler.is_compiling() and not _watched())
 
 
 def fine_loss(ret, target, weight_main=1.0, weight_entropy_last=0.001, weight_rgb0=0.5):
