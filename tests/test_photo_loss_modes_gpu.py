@@ -86,3 +86,21 @@ def test_default_device_keeps_the_kernels(cuda, monkeypatch):
     with torch.device(cuda):
         _loss(fine_loss, xs, target)
     assert used
+
+
+@pytest.mark.parametrize("how", ["is_grads_batched", "vmap", "jacobian"])
+def test_batched_upstream_gradients(cuda, how):
+    """A batch of upstream gradients through one loss: each one's own result."""
+    xs, target = _inputs(5, cuda)
+    ups = torch.tensor([1.0, -2.5, 0.0], device=cuda)
+    want = [torch.autograd.grad(u * _loss(_chain, xs, target), xs) for u in ups]
+    loss = _loss(fine_loss, xs, target)
+    if how == "is_grads_batched":
+        got = torch.autograd.grad(loss, xs, ups, is_grads_batched=True)
+    elif how == "vmap":
+        got = torch.func.vmap(lambda u: torch.autograd.grad(loss, xs, u, retain_graph=True))(ups)
+    else:
+        got = torch.autograd.functional.jacobian(
+            lambda *x: ups * _loss(fine_loss, x, target), tuple(t.detach() for t in xs), vectorize=True)
+    for k in range(3):
+        torch.testing.assert_close(got[k], torch.stack([w[k] for w in want]), rtol=1e-5, atol=1e-9)

@@ -39,9 +39,10 @@ class _PhotoLoss(torch.autograd.Function):
     def backward(ctx, g):
         rgb, rgb0, alphainv, target = ctx.saved_tensors
         w_main, w_rgb0, w_entropy = ctx.weights
-        if torch.is_grad_enabled() or _watched():
-            # create_graph, or a tracer over the backward: the same gradients
-            # from torch operations
+        if torch.is_grad_enabled() or _watched() or _batched(g) or not _plain(g):
+            # create_graph, a tracer over the backward, or upstream gradients
+            # that are no plain tensor (a batch of them, a subclass): the same
+            # gradients from torch operations
             norm = 2.0 / rgb.numel()
             d_rgb = norm * (rgb - target) * (g * w_main)
             d_rgb0 = None if rgb0 is None else norm * (rgb0 - target) * (g * w_rgb0)
@@ -52,7 +53,6 @@ class _PhotoLoss(torch.autograd.Function):
                 d = torch.where((x >= 1e-6) & (x <= 1 - 1e-6), torch.log(1 - p) - torch.log(p), torch.zeros_like(p))
                 d_a = F.pad((g * w_entropy * d)[None], (alphainv.numel() - 1, 0))
             return d_rgb, d_rgb0, d_a, None, None, None, None
-        g = g.contiguous()
         d_rgb = torch.empty_like(rgb)
         d_rgb0 = None if rgb0 is None else torch.empty_like(rgb0)
         d_a = None if alphainv is None else torch.empty_like(alphainv)
@@ -69,6 +69,13 @@ def _last_ptr(t):
 def _plain(t) -> bool:
     return (type(t) is torch.Tensor and t.is_cuda and t.dtype == torch.float32 and t.is_contiguous() and t.numel() > 0
             and not t.is_neg())
+
+
+def _batched(t) -> bool:
+    """Whether t stands for a batch of tensors (vmap, or a backward with
+    is_grads_batched): its type is Tensor, but it has no storage."""
+    c = torch._C._functorch
+    return c.is_functorch_wrapped_tensor(t) or c.is_legacy_batchedtensor(t)
 
 
 def _watched() -> bool:
