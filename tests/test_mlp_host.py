@@ -1,9 +1,10 @@
 """Host logic of the MLP engines: the module and parameter lists they walk."""
 import gc
 
+import torch
 import torch.nn as nn
 
-from voxurf_gb300.mlp import _linears, _modules, _parameters
+from voxurf_gb300.mlp import _grad_buffers, _linears, _modules, _parameters
 
 
 def _stacks():
@@ -32,3 +33,18 @@ def test_walks_leave_no_cycles():
         assert gc.collect() == 0
     finally:
         gc.enable()
+
+
+def test_gradients_are_tensors_of_their_own():
+    """Keeping or saving one gradient keeps no other alive, and changing one in
+    place leaves what autograd saved of the others valid."""
+    lin = _linears(next(_stacks()))
+    grads = _grad_buffers(lin)
+    assert [g.shape for g in grads] == [t.shape for m in lin for t in (m.weight, m.bias)]
+    assert all(g.untyped_storage().nbytes() == 4 * g.numel() for g in grads)
+    assert len({g.untyped_storage().data_ptr() for g in grads}) == len(grads)
+    w = torch.ones_like(grads[2], requires_grad=True)
+    loss = (grads[2].fill_(2.0) * w).sum()
+    grads[3].zero_()
+    loss.backward()
+    assert bool((w.grad == 2.0).all())

@@ -340,13 +340,10 @@ def _parameters(net: nn.Module) -> list:
 
 
 def _grad_buffers(lin: list) -> list[torch.Tensor]:
-    """FP32 gradient buffers [W0, b0, ..., Wh, bh] of Linear layers, parts of
-    one allocation."""
-    shapes = []
-    for m in lin:
-        shapes += [m.weight.shape, m.bias.shape]
-    flat = torch.empty(sum(s.numel() for s in shapes), dtype=torch.float32, device=lin[0].weight.device)
-    return [t if len(s) == 1 else t.view(s) for t, s in zip(flat.split([s.numel() for s in shapes]), shapes)]
+    """FP32 gradient buffers [W0, b0, ..., Wh, bh] of Linear layers, each a
+    tensor of its own: they become the parameters' .grad, and a program may
+    keep, save or change one without the others."""
+    return [torch.empty_like(t) for m in lin for t in (m.weight, m.bias)]
 
 
 class _Scratch:
