@@ -1,9 +1,11 @@
 """Host logic of the MLP engines: the module and parameter lists they walk."""
 import gc
 
+import pytest
 import torch
 import torch.nn as nn
 
+from voxurf_gb300 import _abi, mlp
 from voxurf_gb300.mlp import _grad_buffers, _linears, _modules, _parameters
 
 
@@ -48,3 +50,27 @@ def test_gradients_are_tensors_of_their_own():
     grads[3].zero_()
     loss.backward()
     assert bool((w.grad == 2.0).all())
+
+
+def test_preallocated_buffers_are_checked(monkeypatch):
+    """Buffers made for one row count serve fewer rows, with the capacities
+    they have, and refuse more before anything is launched."""
+    launched = []
+    monkeypatch.setattr(_abi, "call_struct", lambda name, a, st: launched.append((name, a)))
+    monkeypatch.setattr(mlp, "stream_ptr", lambda *a: 0)
+    eng = mlp.TcTrainMLP(nn.Sequential(nn.Linear(20, 32), nn.ReLU(), nn.Linear(32, 32), nn.ReLU(), nn.Linear(32, 3)), 32)
+    saved, work = {}, {}
+
+    def one_pass(n, saved, work):
+        x = torch.zeros((n, 32), dtype=torch.bfloat16)
+        _, st = eng.forward(x, saved=saved)
+        return eng.backward_chain(st, torch.zeros((n, 3)), work=work)[2]
+
+    caps = [g.part_cap for g, *_ in one_pass(40_000, saved, work)]
+    assert [g.part_cap for g, *_ in one_pass(500, saved, work)] == caps
+    launched.clear()
+    with pytest.raises(ValueError, match="too small"):
+        one_pass(40_200, saved, {})
+    with pytest.raises(ValueError, match="too small"):
+        one_pass(40_200, {}, work)
+    assert [name for name, _ in launched] == ["vx_mlp_train_forward"]   # the second one's own

@@ -347,20 +347,24 @@ def _grad_buffers(lin: list) -> list[torch.Tensor]:
 
 
 class _Scratch:
-    """One allocation for several buffers of an engine: `take` hands out
-    256-byte aligned offsets, `alloc` makes the bytes.  Seven torch.empty calls
-    cost more host time than the kernels of a small batch."""
+    """One allocation for the buffers of an engine, `sizes` bytes each at
+    256-byte aligned offsets.  Seven torch.empty calls cost more host time than
+    the kernels of a small batch."""
 
-    def __init__(self):
-        self.nbytes = 0
+    def __init__(self, sizes, device):
+        self.sizes, self.at, n = list(sizes), [], 0
+        for s in self.sizes:
+            self.at.append(n)
+            n = _round_up(n + s, 256)
+        self.buf = torch.empty(max(n, 16), dtype=torch.uint8, device=device)
 
-    def take(self, nbytes: int) -> int:
-        at = self.nbytes
-        self.nbytes = _round_up(at + nbytes, 256)
-        return at
-
-    def alloc(self, device) -> torch.Tensor:
-        return torch.empty(max(self.nbytes, 16), dtype=torch.uint8, device=device)
+    def ptrs(self, sizes) -> list[int]:
+        """The buffers' addresses for a pass that needs `sizes` bytes of them;
+        a pass on more rows than they were made for is refused."""
+        if len(sizes) != len(self.sizes) or any(s > have for s, have in zip(sizes, self.sizes)):
+            raise ValueError("preallocated MLP buffers are too small for these rows")
+        base = self.buf.data_ptr()
+        return [base + o for o in self.at]
 
 
 class TcTrainMLP:
@@ -445,6 +449,10 @@ class TcTrainMLP:
         """FP32 gradient buffers in parameter order [W0, b0, ..., Wh, bh]."""
         return _grad_buffers(self.lin)
 
+    def _saved_bytes(self, cap: int) -> tuple:
+        """Hidden T-tiles and ReLU bits of `cap` rows."""
+        return self.L * cap * self.W * 2, self.L * cap * (self.W // 16) * 2
+
     def forward(self, X: torch.Tensor, out: torch.Tensor | None = None, train: bool = True,
                 cols: torch.Tensor | None = None, n_rows_dev: torch.Tensor | None = None,
                 saved: dict | None = None) -> tuple[torch.Tensor, dict | None]:
@@ -464,10 +472,9 @@ class TcTrainMLP:
         st = None
         if train:
             st = saved if saved is not None else {}
+            sizes = self._saved_bytes(cap)
             if "buf" not in st:
-                sc = _Scratch()
-                st["at"] = (sc.take(self.L * cap * self.W * 2), sc.take(self.L * cap * (self.W // 16) * 2))
-                st["buf"] = sc.alloc(dev)   # hidden T-tiles, ReLU bits
+                st["buf"] = _Scratch(sizes, dev)
             st["cap"], st["n"], st["X"], st["n_rows_dev"] = cap, n, X, n_rows_dev
         a = _abi.MlpTrainFwdArgs()
         a.n_rows, a.n_rows_dev, a.rows_cap = n, ptr(n_rows_dev), cap
@@ -479,7 +486,7 @@ class TcTrainMLP:
             raise ValueError("cols must be BF16 for BF16 rows")
         a.cols, a.ld_cols = ptr(cols), (cols.stride(0) if cols is not None else 0)
         if train:
-            a.H, a.relu = (st["buf"].data_ptr() + o for o in st["at"])
+            a.H, a.relu = st["buf"].ptrs(sizes)
         _abi.call_struct("vx_mlp_train_forward", a, stream_ptr(dev))
         return out, st
 
@@ -510,15 +517,14 @@ class TcTrainMLP:
             raise ValueError("dY must be contiguous FP32 [n, 3]")
         grid = int(lib.vx_mlp_wgrad_grid(n))
         w = work if work is not None else {}
+        # dz T-tiles, dy T-tiles, column sums of dy, weight-gradient partials
+        sizes = [L * cap * W * 2, cap * 16 * 2, grid * 4 * 4, grid * W * (K0 + 16) * 4, grid * W * 16 * 4]
+        sizes += [grid * W * (W + 16) * 4] * (L - 1)
         if "buf" not in w:
-            # dz T-tiles, dy T-tiles, column sums of dy, weight-gradient partials
-            sc = _Scratch()
-            offs = [sc.take(L * cap * W * 2), sc.take(cap * 16 * 2), sc.take(grid * 4 * 4),
-                    sc.take(grid * W * (K0 + 16) * 4), sc.take(grid * W * 16 * 4)]
-            offs += [sc.take(grid * W * (W + 16) * 4) for _ in range(L - 1)]
-            w["buf"], w["at"] = sc.alloc(dev), offs
-        dZ, dYT, dbh, part0, parth, *part = (w["buf"].data_ptr() + o for o in w["at"])
-        H, relu = (st["buf"].data_ptr() + o for o in st["at"])
+            w["buf"] = _Scratch(sizes, dev)
+        dZ, dYT, dbh, part0, parth, *part = w["buf"].ptrs(sizes)
+        part0_cap, parth_cap, *part_cap = (s // 4 for s in w["buf"].sizes[3:])
+        H, relu = st["buf"].ptrs(self._saved_bytes(cap))
         if dX is None:
             dX = torch.empty((n, K0), dtype=dx_dtype, device=dev)
         if grads is None:
@@ -535,21 +541,21 @@ class TcTrainMLP:
         R = _abi.MlpReduceJob
         pending = []   # (pass arguments, reduce job of its n_part partials, the buffers both point into)
 
-        def wgrad(A, WA, B, WB, ldb, b_rows, ones, part, job):
+        def wgrad(A, WA, B, WB, ldb, b_rows, ones, part, cap, job):
             g = _abi.MlpWgradArgs()
             g.n_rows, g.n_rows_dev, g.A, g.WA, g.B, g.WB, g.ldb = n, ptr(st["n_rows_dev"]), A, WA, B, WB, ldb
-            g.b_rows, g.ones, g.part, g.part_cap = b_rows, ones, part, grid * WA * (WB + 16 * ones)
+            g.b_rows, g.ones, g.part, g.part_cap = b_rows, ones, part, cap
             pending.append((g, job, (w["buf"], st["buf"], X)))
 
         for l in range(1, L):   # dW_l = dz_{l+1}^T h_l
             pl = part[l - 1]
-            wgrad(dZ + l * lay, W, H + (l - 1) * lay, W, 0, 0, 1, pl,
+            wgrad(dZ + l * lay, W, H + (l - 1) * lay, W, 0, 0, 1, pl, part_cap[l - 1],
                   lambda k, pl=pl, l=l: R(pl, k, W, W + 16, 0, 0, W, W, grads[2 * l].data_ptr(),
                                           grads[2 * l + 1].data_ptr(), None, 0))
-        wgrad(dZ, W, X.data_ptr(), K0, X.stride(0), 1, 1, part0,      # dW_0 = dz_1^T X
+        wgrad(dZ, W, X.data_ptr(), K0, X.stride(0), 1, 1, part0, part0_cap,      # dW_0 = dz_1^T X
               lambda k: R(part0, k, W, K0 + 16, 0, 0, K0, self.d_in, grads[0].data_ptr(),
                           grads[1].data_ptr(), None, 0))
-        wgrad(H + (L - 1) * lay, W, dYT, 16, 0, 0, 0, parth,   # dWh = dy^T h_L
+        wgrad(H + (L - 1) * lay, W, dYT, 16, 0, 0, 0, parth, parth_cap,   # dWh = dy^T h_L
               lambda k: R(parth, k, W, 16, 1, 0, 16, 3, grads[2 * L].data_ptr(),
                           grads[2 * L + 1].data_ptr(), dbh, grid))
         return dX, grads, pending
