@@ -16,46 +16,57 @@
 // Segment bounds come from a search in the sorted ray_id instead of the
 // reference's scatter kernel + device-indexed host write (:607-635).
 //
-// Bound: the latency of a ray's chain (search, loads, scans); the bytes (24
-// a sample forward, 24 backward) would take 14 us at 8192 rays x 400
-// samples.  Forward and backward there, with the host's two calls: 178 us
-// with 32 samples a step, a bisection per bound and FP64 beyond 512 samples
-// (62 + 105 us of kernels), 74 us now, where the calls themselves take as
-// long as the kernels.
+// Bound: the latency of a ray's chain (search, loads, scans).  At 8192 rays x
+// 400 samples every input read and every output written once (alpha, ray_id,
+// grad_weights in; weight, T, grad out: 28 bytes a sample) would take 14 us;
+// the two kernels move 36 (12 forward, where ray_id is only probed, and 24
+// backward, which reads weight and T again and clears grad first): 17 us.
+// Forward and backward there, with the host's two calls: 178 us with 32
+// samples a step, a bisection per bound and FP64 beyond 512 samples (62 + 105
+// us of kernels), 74 us now, where the calls themselves take as long as the
+// kernels.
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace vx {
 
 // Segment [beg, end) of ray r in a sorted ray_id array.  Each half of the
 // warp searches one bound, sixteen probes a step: six dependent loads for
-// millions of samples, where a bisection takes 22.
+// millions of samples, where a bisection takes 22.  The probes are 1/16 of the
+// range and one sample apart: a shift, where sixteen even parts of it took
+// 64-bit divisions that cost a million short rays more than they saved.
 __device__ __forceinline__ void ray_segment(const int64_t* __restrict__ ray_id, int64_t n_pts, int64_t r,
                                             int64_t* beg, int64_t* end) {
   const int lane = lane_id(), half = lane >> 4, sub = lane & 15;
   const int64_t key = r + half;
   int64_t lo = 0, hi = n_pts;
   while (__any_sync(0xffffffffu, lo < hi)) {
-    const int64_t n = hi - lo;
-    // n * (sub + 1) / 17 without the overflow, always below n
-    const int64_t at = lo + n / 17 * (sub + 1) + n % 17 * (sub + 1) / 17;
-    const bool less = lo < hi && ray_id[at] < key;
+    const int64_t step = ((hi - lo) >> 4) + 1;             // 16 steps reach past hi
+    const int64_t at = lo + step * (sub + 1) - 1;
+    const bool less = at < hi && ray_id[at] < key;
     const int c = __popc((__ballot_sync(0xffffffffu, less) >> (16 * half)) & 0xffffu);
-    const int64_t below = __shfl_sync(0xffffffffu, at, 16 * half + max(c - 1, 0));
-    const int64_t above = __shfl_sync(0xffffffffu, at, 16 * half + min(c, 15));
-    if (lo < hi) {
-      if (c > 0) lo = below + 1;
-      if (c < 16) hi = above;
-    }
+    lo = min(lo + step * c, hi);                           // (beyond hi only where ray_id is not sorted)
+    hi = min(hi, lo + step - 1);
   }
   *beg = __shfl_sync(0xffffffffu, lo, 0);
   *end = __shfl_sync(0xffffffffu, lo, 16);
 }
 
-constexpr int CHUNKS = 4;   // 32-sample scans in flight per warp
+// 32-sample scans in flight per warp: as many as the segment fills, up to
+// four.  (Four for every segment: 1M rays of 1 to 5 samples 803 us forward and
+// 327 us backward with the even search above, where one scan and a bisection
+// took 667 and 278.)
+template <typename F>
+__device__ __forceinline__ void by_chunks(int64_t len, F scan) {
+  if (len <= 32) scan(std::integral_constant<int, 1>());
+  else if (len <= 64) scan(std::integral_constant<int, 2>());
+  else scan(std::integral_constant<int, 4>());
+}
 
 // Warp-level forward scan of one segment.  Writes weight/T for every sample
 // of [beg, end); returns i_end and alphainv_last in every lane.
-template <typename Acc>
+template <typename Acc, int CHUNKS>
 __device__ __forceinline__ void scan_segment_fwd(const float* __restrict__ alpha, int64_t beg, int64_t end,
                                                  float* __restrict__ weight, float* __restrict__ T,
                                                  int64_t* i_end_out, float* last_out) {
@@ -133,9 +144,9 @@ __global__ void alpha2weight_kernel(const float* __restrict__ alpha, const int64
   int64_t ie;
   float last;
   if (end - beg > VX_FP32_SCAN_MAX_STEPS)
-    scan_segment_fwd<FloatPair>(alpha, beg, end, weight, T, &ie, &last);
+    scan_segment_fwd<FloatPair, 4>(alpha, beg, end, weight, T, &ie, &last);
   else
-    scan_segment_fwd<float>(alpha, beg, end, weight, T, &ie, &last);
+    by_chunks(end - beg, [&](auto c) { scan_segment_fwd<float, c>(alpha, beg, end, weight, T, &ie, &last); });
   if (lane_id() == 0) {
     i_start[r] = beg;
     i_end[r] = ie;
@@ -148,7 +159,7 @@ __global__ void alpha2weight_kernel(const float* __restrict__ alpha, const int64
 //     grad[i] = gw[i]*T[i] - back/(1-alpha[i]+1e-10);  back += gw[i]*w[i]
 // The running sum `back` is carried in Acc (a FloatPair on segments of more
 // than 512 samples).
-template <typename Acc>
+template <typename Acc, int CHUNKS>
 __device__ __forceinline__ void scan_segment_bwd(const float* __restrict__ alpha, const float* __restrict__ weight,
                                                  const float* __restrict__ T, const float* __restrict__ grad_w,
                                                  int64_t beg, int64_t end, float back0,
@@ -209,9 +220,11 @@ __global__ void alpha2weight_backward_kernel(const float* __restrict__ alpha, co
     return;
   }
   if (end - beg > VX_FP32_SCAN_MAX_STEPS)
-    scan_segment_bwd<FloatPair>(alpha, weight, T, grad_weights, beg, end, grad_last[r] * alphainv_last[r], grad);
+    scan_segment_bwd<FloatPair, 4>(alpha, weight, T, grad_weights, beg, end, grad_last[r] * alphainv_last[r], grad);
   else
-    scan_segment_bwd<float>(alpha, weight, T, grad_weights, beg, end, grad_last[r] * alphainv_last[r], grad);
+    by_chunks(end - beg, [&](auto c) {
+      scan_segment_bwd<float, c>(alpha, weight, T, grad_weights, beg, end, grad_last[r] * alphainv_last[r], grad);
+    });
 }
 
 }  // namespace vx
