@@ -260,10 +260,11 @@ __global__ void __launch_bounds__(SM_THREADS, 3) smooth_march_kernel(const float
   cp_async_wait_group<0>();
 }
 
-// The same sweep without shared memory, for rows of whole float4s (Z % 4 == 0,
-// 16-byte aligned buffers) and up to five taps: a warp owns 4 (y) x 128 (z)
-// outputs of a chunk of x and a lane four consecutive z.  It reads the 4 + 2H
-// rows of a plane as float4s, takes the z neighbours of a lane's four values by
+// The same sweep without passes through shared memory, for rows of whole
+// float4s (Z % 4 == 0, 16-byte aligned buffers) and up to five taps: a warp owns
+// 4 (y) x 128 (z) outputs of a chunk of x and a lane four consecutive z.  It
+// reads the 4 + 2H rows of a plane as float4s (cp.async into the lane's own
+// 16 bytes of shared memory, no barrier: 49 KB a block for five taps), takes the z neighbours of a lane's four values by
 // shuffle (the two lanes at the tile's ends by a load of their own), runs the y
 // pass over the rows in registers and keeps the last 2H + 1 y-passed planes for
 // the x pass; the plane loop is unrolled 2H + 1 times, so the ring needs no
@@ -271,8 +272,8 @@ __global__ void __launch_bounds__(SM_THREADS, 3) smooth_march_kernel(const float
 // the same products in the same order as the kernel above: the bits are equal.
 // Bound: L2 reads (each row is read by two warps) and their latency; 74 thread
 // instructions an output became about 20.  The planes arrive by cp.async, three
-// deep.  256^3, five taps, cold L2: forward 56 -> 37 us, adjoint 76 -> 50 us (20 us
-// of HBM); 384^3 146 -> 120 and 218 -> 173 us.
+// deep.  Five taps, inputs from HBM: 256^3 forward 55 -> 36 us, adjoint 77 -> 50 us
+// (20 us of HBM); 384^3 149 -> 101 and 221 -> 138 us.
 constexpr int SR_WARPS = 4;      // consecutive y tiles share rows through L1
 constexpr int SR_Z = 128;
 constexpr int SR_STAGES = 3;     // planes on their way or in use
@@ -511,15 +512,21 @@ __global__ void __launch_bounds__(32 * SR_WARPS, 3) smooth_rows_kernel(const flo
   }
 }
 
-// x chunking: about twelve warps a multiprocessor, chunks of >= 8 planes
-// (each reads 2H more than it writes).
+// x chunking: the number of chunks (of >= 8 planes; each reads 2H more than it
+// writes) whose waves of three CTAs a multiprocessor pass the fewest planes.
+// (Twelve warps a multiprocessor rounded up to whole chunks left a second wave
+// with a few CTAs: 512 x 512 x 132 adjoint 192 us, 146 now.)
 template <bool ADJOINT, bool ACCUM, int H>
 static int launch_rows(const float* in, float* out, int X, int Y, int Z, const Taps& t, cudaStream_t st) {
   const int n_yt = (Y + 4 * SR_WARPS - 1) / (4 * SR_WARPS), n_zt = (Z + SR_Z - 1) / SR_Z;
-  const int64_t want = (int64_t)sm_count() * 12 / SR_WARPS;
-  int64_t n_xc = (want + (int64_t)n_yt * n_zt - 1) / ((int64_t)n_yt * n_zt);
-  n_xc = std::max<int64_t>(1, std::min<int64_t>(n_xc, (X + 7) / 8));
-  const int CX = (int)((X + n_xc - 1) / n_xc);
+  const int64_t slots = (int64_t)sm_count() * 3, tiles = (int64_t)n_yt * n_zt;
+  int CX = X;
+  int64_t best = INT64_MAX;
+  for (int n = 1; n <= (X + 7) / 8; ++n) {
+    const int cx = (X + n - 1) / n, n_xc = (X + cx - 1) / cx;
+    const int64_t cost = (tiles * n_xc + slots - 1) / slots * (cx + 2 * H);
+    if (cost < best) best = cost, CX = cx;
+  }
   const dim3 grid((unsigned)n_yt, (unsigned)n_zt, (unsigned)((X + CX - 1) / CX));
   auto kernel = smooth_rows_kernel<ADJOINT, ACCUM, H>;
   const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SrGeom<H>::SMEM);
@@ -545,13 +552,26 @@ static int launch_march(const float* in, float* out, int X, int Y, int Z, const 
   return launch_status();
 }
 
+// Where the row kernel is the faster one.  Below 128^3 it has too few warps to
+// hide its loads (96^3 forward 15 against 13 us).  Its tile is 128 z wide and the
+// other's 32: a single tile pays from 33 z on forward (512 x 512 x 32: 50 against
+// 32 us, x 36: 50 against 92) and from 65 on in the adjoint (x 64: 82 against 78,
+// x 80: 82 against 97), and an adjoint whose last tile holds no more than 32
+// pays from about three million voxels on (100 x 200 x 140: 22.5 against 21 us,
+// 148^3: 23 against 31, 512 x 512 x 132: 146 against 176).
+template <bool ADJOINT>
+static bool takes_rows(int X, int Y, int Z) {
+  const int64_t voxels = (int64_t)X * Y * Z;
+  const int tail = Z % SR_Z;
+  if (Z % 4 || std::min(X, std::min(Y, Z)) <= 4 || (Z + SR_Z - 1) / SR_Z > 65535 || (X + 7) / 8 > 65535) return false;
+  if (ADJOINT) return Z > 64 && voxels >= (tail > 0 && tail <= 32 ? 3 << 20 : 1 << 21);
+  return Z > 32 && voxels >= 1 << 21;
+}
+
 template <bool ADJOINT, bool ACCUM>
 static int launch_h(const float* in, float* out, int X, int Y, int Z, const Taps& t, cudaStream_t st) {
-  // below 128^3 the row kernel has too few warps to hide its loads (96^3
-  // forward 15 against 13 us); from there on it is the faster one (128^3 19
-  // against 21 us adjoint, 256^3 50 against 76)
-  const bool rows = (int64_t)X * Y * Z >= 128 * 128 * 128 && Z % 4 == 0 && ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15) == 0 &&
-                    std::min(X, std::min(Y, Z)) > 4 && (Z + SR_Z - 1) / SR_Z <= 65535 && (X + 7) / 8 <= 65535;
+  const bool rows = takes_rows<ADJOINT>(X, Y, Z) &&
+                    ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
   if (rows && t.h <= 2) {
     if (t.h == 0) return launch_rows<ADJOINT, ACCUM, 0>(in, out, X, Y, Z, t, st);
     if (t.h == 1) return launch_rows<ADJOINT, ACCUM, 1>(in, out, X, Y, Z, t, st);
