@@ -28,7 +28,6 @@ namespace mf {
 
 constexpr int BM = 64;          // rows per rowgemm tile
 constexpr int RG_THREADS = 128; // 8 x 16 threads
-constexpr int RG_M = BM / 8;    // rows per thread
 constexpr int KC = 16;          // K per shared-memory stage
 constexpr int THREADS = 256;    // weight gradient: 16 x 16 threads
 
@@ -64,9 +63,11 @@ constexpr int AS_LD = KC + 4;  // A stage row stride (floats): 16-byte rows, no 
 // below them: with 4 x 12 outputs a thread the reads of Bt took 81% of the L1
 // cycles.  131,003 rows: five layers (K = 70 and 192, N = 192) 1,039 us with
 // scalar products and 4 x 12 outputs a thread, 853 us now (57 TFLOP/s).
-template <int TN>
+// A tile is RM x 8 rows: 64, or 32 where 64-row tiles would leave CTAs without
+// one (the sums are the same bits).
+template <int TN, int RM>
 __global__ void __launch_bounds__(RG_THREADS, 3) rowgemm_kernel(RowGemmParams P) {
-  constexpr int NP = 16 * TN;
+  constexpr int NP = 16 * TN, BM = 8 * RM, RG_M = RM;
   // dynamic shared memory: the A ring, the Bt ring; the column-sum scratch of
   // the epilogue reuses the A ring
   extern __shared__ __align__(16) float rg_smem[];
@@ -460,19 +461,27 @@ int vx_mlp_f32_rowgemm(const vx_mlp_f32_rowgemm_args* a, void* stream) {
   const unsigned grid = (unsigned)vx_mlp_f32_rowgemm_grid(a->M);
   cudaStream_t st = as_stream(stream);
   if (split_rowgemm_takes(P)) return split_rowgemm_launch(P, st);
-  auto launch = [&](auto kernel, int np) -> int {
-    const size_t smem = sizeof(float) * ((size_t)RG_STAGES * BM * AS_LD + (size_t)RG_STAGES * KC * np);
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  // While 64-row tiles leave multiprocessors without one, 32-row tiles (not in
+  // mode 1, whose column sums are laid out by 64-row tiles): three 192-wide
+  // layers forward take 71 us with 64-row tiles at 5,000 rows and 67 at 2,000, 65
+  // and 50 with 32.
+  const bool small = a->mode != 1 && (int64_t)grid < sm_count();
+  auto go = [&](auto kernel, int bm, int np) -> int {
+    const size_t smem = sizeof(float) * ((size_t)RG_STAGES * bm * AS_LD + (size_t)RG_STAGES * KC * np);
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return cuda_status(e);
-    kernel<<<grid, RG_THREADS, smem, st>>>(P);
+    kernel<<<(unsigned)std::max<int64_t>(1, (a->M + bm - 1) / bm), RG_THREADS, smem, st>>>(P);
     return launch_status();
   };
+  auto launch = [&](auto kernel, auto kernel_small, int np) -> int {
+    return small ? go(kernel_small, BM / 2, np) : go(kernel, BM, np);
+  };
   switch (a->Np) {
-    case 32: return launch(rowgemm_kernel<2>, 32);
-    case 64: return launch(rowgemm_kernel<4>, 64);
-    case 80: return launch(rowgemm_kernel<5>, 80);
-    case 128: return launch(rowgemm_kernel<8>, 128);
-    case 192: return launch(rowgemm_kernel<12>, 192);
+    case 32: return launch(rowgemm_kernel<2, 8>, rowgemm_kernel<2, 4>, 32);
+    case 64: return launch(rowgemm_kernel<4, 8>, rowgemm_kernel<4, 4>, 64);
+    case 80: return launch(rowgemm_kernel<5, 8>, rowgemm_kernel<5, 4>, 80);
+    case 128: return launch(rowgemm_kernel<8, 8>, rowgemm_kernel<8, 4>, 128);
+    case 192: return launch(rowgemm_kernel<12, 8>, rowgemm_kernel<12, 4>, 192);
     default: return VX_ERR_UNSUPPORTED;
   }
 }
