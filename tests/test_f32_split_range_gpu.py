@@ -1,0 +1,35 @@
+"""The split-operand backward GEMMs at the ends of FP32's range, against the
+CUDA-core kernels (an odd row stride sends a call there) and 64 bits."""
+import pytest
+import torch
+
+from test_f32_split_gpu import _err, _rowgemm, _rows, _wgrad
+
+pytestmark = pytest.mark.gpu
+
+
+def _bits(x):
+    return x.view(torch.int32)
+
+
+# products that overflow although each operand is far from it, with both signs
+# of the parts after the first (1.003 and 0.999 round down and up to BF16)
+@pytest.mark.parametrize("a,b", [(1.003e25, 1.003e25), (0.999e25, 1.003e25), (1.003e25, -0.999e25), (3e19, 3e19),
+                                 (1.003e30, 1.003e12)])
+def test_products_that_overflow(cuda, a, b):
+    n = 400
+    A = torch.randn((n, 192), generator=torch.Generator().manual_seed(0)).to(cuda)
+    B = torch.randn((n, 192), generator=torch.Generator().manual_seed(1)).to(cuda)
+    A[150, 7], B[150, 20] = a, b
+    split, plain = (_wgrad(_rows(A, 192 + p), _rows(B, 192 + p), 192, 192) for p in (0, 1))
+    torch.testing.assert_close(split, plain, rtol=1e-4, atol=1e-4 * max(abs(a), abs(b)))
+    big = ~plain.isfinite()
+    assert torch.equal(_bits(split)[big], _bits(plain)[big]) and not split.isnan().any()
+    Bt = torch.randn((192, 192), generator=torch.Generator().manual_seed(2)).to(cuda)
+    Bt[7, 100] = b
+    split, plain = (_rowgemm(_rows(A, 192 + p), Bt)[0] for p in (0, 1))
+    big = ~plain.isfinite()
+    assert torch.equal(_bits(split)[big], _bits(plain)[big]) and not split.isnan().any()
+    # every other sum: rounding of its largest products
+    scale = A.abs().double() @ Bt.abs().double()
+    assert bool(((split.double() - plain.double()).abs()[~big] <= 192 * 2.0 ** -23 * scale[~big]).all())

@@ -16,10 +16,10 @@
 // The forward keeps its CUDA-core sums: a ReLU whose input lies within a
 // rounding of zero would switch with them.
 //
-// A value that has no such parts (infinite, NaN, or so large that bf16(x)
-// overflows) is noticed while it is split; the tile or the CTA's partial that
-// holds one is computed again by plain FP32 sums, as the CUDA-core kernels
-// form them.
+// A value that has no such parts (infinite or NaN), or one so large that a
+// product with another could overflow (hi hi to +inf beside hi mid to -inf), is
+// noticed while it is split; the tile or the CTA's partial that holds one is
+// computed again by plain FP32 sums, as the CUDA-core kernels form them.
 //
 //   split_rowgemm_kernel  C = A Bt (dz_l = (dz_{l+1} W_l) * [h_l > 0] with the
 //                         column sums of the bias gradient; dX = dz_1 W_0):
@@ -50,7 +50,7 @@ using bf16 = __nv_bfloat16;
 
 constexpr int SP_THREADS = 512;     // 16 warps: TMEM lane quarter = warp % 4, column part = warp / 4
 constexpr int TILE_M = 128;
-constexpr float SPLIT_MAX = 1e38f;  // below it hi, mid and lo are finite
+constexpr float SPLIT_MAX = 0x1p58f;  // below it no product overflows, nor the sum of 1,024 of them
 
 // The parts of two neighbouring values, packed (the first in the lower half).
 struct Split2 {
