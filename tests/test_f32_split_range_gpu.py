@@ -33,3 +33,33 @@ def test_products_that_overflow(cuda, a, b):
     # every other sum: rounding of its largest products
     scale = A.abs().double() @ Bt.abs().double()
     assert bool(((split.double() - plain.double()).abs()[~big] <= 192 * 2.0 ** -23 * scale[~big]).all())
+
+
+@pytest.mark.parametrize("a,b", [(1e-36, 1.0), (1.0, 1e-36), (3e-34, 1.0), (1e-30, 1e-3), (1e-20, 1e-17)])
+def test_tiny_operands_no_less_exact_than_cuda_cores(cuda, a, b):
+    """Values whose second and third BF16 parts would be below BF16's range."""
+    g = torch.Generator().manual_seed(4)
+    A = (a * torch.randn((3000, 192), generator=g)).to(cuda)
+    Bt = (b / 14 * torch.randn((192, 192), generator=g)).to(cuda)
+    split, plain = (_rowgemm(_rows(A, 192 + p), Bt)[0] for p in (0, 1))
+    ref = A.double() @ Bt.double()
+    e = _err(split, ref), _err(plain, ref)
+    print("rows %.3g %.3g" % e)
+    assert e[0] <= e[1]
+    B = (b * torch.randn((3000, 192), generator=g)).to(cuda)
+    split, plain = (_wgrad(_rows(A, 192 + p), _rows(B, 192 + p), 192, 192) for p in (0, 1))
+    ref = A.double().t() @ B.double()
+    e = [_err(x.double().sum(0), ref) for x in (split, plain)]
+    print("wgrad %.3g %.3g" % tuple(e))
+    assert e[0] <= e[1]
+
+
+def test_tiny_rows_among_others(cuda):
+    """Each row is as exact as its own magnitude asks, also beside larger ones."""
+    g = torch.Generator().manual_seed(5)
+    A = (torch.randn((4000, 192), generator=g) * 10.0 ** -torch.randint(0, 37, (4000, 1), generator=g)).to(cuda)
+    Bt = (torch.randn((192, 192), generator=g) / 14).to(cuda)
+    ref = A.double() @ Bt.double()
+    r = [((x.double() - ref).norm(dim=1) / ref.norm(dim=1)).quantile(0.99).item()
+         for x in (_rowgemm(_rows(A, 192 + p), Bt)[0] for p in (0, 1))]
+    assert r[0] <= 1.1 * r[1], r

@@ -2,7 +2,10 @@
 // parts each, FP32 accumulation kept as exact as the CUDA-core sums.
 //
 // x = hi + mid + lo with hi = bf16(x), mid = bf16(x - hi), lo = bf16(x - hi -
-// mid): 3 x 8 significant bits, all 24 of an FP32 value.  a b is summed as the
+// mid): 3 x 8 significant bits, all 24 of an FP32 value.  The operands are
+// scaled by 2^24 first (and the sums by 2^-48), so that the parts of the smallest
+// value, subnormals included, are normal BF16 numbers: unscaled, lo and then mid
+// of a value below about 2^-110 fall under BF16's smallest.  a b is summed as the
 // six products hi hi, hi mid, mid hi, mid mid, hi lo, lo hi; the three dropped
 // ones are below 2^-24 of it.  A product of BF16 values is exact, but each MMA
 // (16 k) truncates its running FP32 sum once.  So
@@ -50,9 +53,12 @@ using bf16 = __nv_bfloat16;
 
 constexpr int SP_THREADS = 512;     // 16 warps: TMEM lane quarter = warp % 4, column part = warp / 4
 constexpr int TILE_M = 128;
-constexpr float SPLIT_MAX = 0x1p58f;  // below it no product overflows, nor the sum of 1,024 of them
+constexpr float SCALE = 0x1p24f;      // of the operands before they are split
+constexpr float UNSCALE = 0x1p-48f;   // of the sums of their products
+constexpr float SPLIT_MAX = 0x1p34f;  // below it no scaled product overflows, nor the sum of 1,024 of them
 
-// The parts of two neighbouring values, packed (the first in the lower half).
+// The parts of two neighbouring values times SCALE, packed (the first in the
+// lower half).
 struct Split2 {
   uint32_t hi, mid, lo;
 };
@@ -63,6 +69,8 @@ __device__ __forceinline__ float bf16_hi(uint32_t p) { return __uint_as_float(p 
 __device__ __forceinline__ Split2 split2(float a, float b, bool& bad) {
   Split2 s;
   bad |= !(fabsf(a) < SPLIT_MAX) || !(fabsf(b) < SPLIT_MAX);
+  a *= SCALE;
+  b *= SCALE;
   s.hi = pack_bf16(a, b);
   a -= bf16_lo(s.hi);
   b -= bf16_hi(s.hi);
@@ -321,7 +329,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1) split_rowgemm_kernel(RowGemmPar
         float v[2];
 #pragma unroll
         for (int e = 0; e < 2; ++e)
-          v[e] = __uint_as_float(ds[i >> 1][2 * (i & 1) + e]) + __uint_as_float(dh[i >> 1][2 * (i & 1) + e]);
+          v[e] = UNSCALE * (__uint_as_float(ds[i >> 1][2 * (i & 1) + e]) + __uint_as_float(dh[i >> 1][2 * (i & 1) + e]));
         if (row >= M) continue;
         if (P.mode == 1) {
           const int bit = 8 * j + 2 * i;
@@ -533,7 +541,8 @@ __global__ void __launch_bounds__(WgradGeo<M, NC>::THREADS + 32, 1) split_wgrad_
         ld_cols<16>(tm_lanes + (uint32_t)(mt * NC + c), s);
         ld_cols<16>(tm_lanes + (uint32_t)(G::D_HI + mt * NC + c), h);
 #pragma unroll
-        for (int e = 0; e < 16; ++e) acc[mt][b][e] += __uint_as_float(s[e]) + __uint_as_float(h[e]);
+        for (int e = 0; e < 16; ++e)
+          acc[mt][b][e] = fmaf(UNSCALE, __uint_as_float(s[e]) + __uint_as_float(h[e]), acc[mt][b][e]);
       }
     }
   };
