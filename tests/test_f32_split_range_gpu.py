@@ -4,6 +4,8 @@ import pytest
 import torch
 
 from test_f32_split_gpu import _err, _rowgemm, _rows, _wgrad
+from voxurf_gb300 import _abi
+from voxurf_gb300._torch import ptr, stream_ptr
 
 pytestmark = pytest.mark.gpu
 
@@ -63,3 +65,40 @@ def test_tiny_rows_among_others(cuda):
     r = [((x.double() - ref).norm(dim=1) / ref.norm(dim=1)).quantile(0.99).item()
          for x in (_rowgemm(_rows(A, 192 + p), Bt)[0] for p in (0, 1))]
     assert r[0] <= 1.1 * r[1], r
+
+
+def _reduced(part):
+    """The engine's own ordered sum of the partials."""
+    grid, M, N = part.shape
+    part, out = part.contiguous(), torch.empty((M, N), device=part.device)
+    job = _abi.MlpSumJob(ptr(part), grid, M * N, N, M, N, ptr(out), N)
+    _abi.call("vx_mlp_f32_reduce", (_abi.MlpSumJob * 1)(job), 1, stream_ptr(part.device))
+    return out
+
+
+@pytest.mark.parametrize("rows", [33, 65, 700, 60_001, 131_003])
+@pytest.mark.parametrize("M,N,NP", [(192, 192, 192), (128, 60, 64)])
+def test_wgrad_of_one_sign(cuda, M, N, NP, rows):
+    """Products of one sign, whose sums truncation always leaves short: the
+    gradient that the engine returns is as exact as the CUDA-core kernels'.
+    (Both end in the same ordered FP32 sum of up to 152 partials, about 5e-8;
+    a tenth is left for which way its roundings fall.)"""
+    g = torch.Generator().manual_seed(rows)
+    A, B = torch.rand((rows, M), generator=g).to(cuda), torch.rand((rows, N), generator=g).to(cuda)
+    ref = A.double().t() @ B.double()
+    e = [_err(_reduced(_wgrad(_rows(A, M + p), _rows(B, (N + 3) // 4 * 4 + p), M, NP)), ref) for p in (0, 1)]
+    print(M, N, rows, "%.3g %.3g" % tuple(e))
+    assert e[0] <= max(1.1 * e[1], 2.0 ** -24)
+
+
+def test_rowgemm_of_one_sign(cuda):
+    """Rows are more exact than the CUDA-core kernels' here too; their column
+    sums keep the truncation of 8 and 4 MMAs: at most (4.5 * 2 / 3 + 2.5 / 3)
+    units of 2^-23, half of it on average."""
+    g = torch.Generator().manual_seed(6)
+    A, Bt = torch.rand((60_001, 192), generator=g).to(cuda), torch.rand((192, 192), generator=g).to(cuda)
+    H = torch.ones((A.shape[0], 192), device=cuda)
+    ref = A.double() @ Bt.double()
+    (split, sums), (plain, _) = (_rowgemm(_rows(A, 192 + p), Bt, H) for p in (0, 1))
+    assert _err(split, ref) <= _err(plain, ref)
+    assert _err(sums.double().sum(0), ref.sum(0)) <= 3.9 / 2 * 2.0 ** -23
