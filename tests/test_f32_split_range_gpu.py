@@ -102,3 +102,31 @@ def test_rowgemm_of_one_sign(cuda):
     (split, sums), (plain, _) = (_rowgemm(_rows(A, 192 + p), Bt, H) for p in (0, 1))
     assert _err(split, ref) <= _err(plain, ref)
     assert _err(sums.double().sum(0), ref.sum(0)) <= 3.9 / 2 * 2.0 ** -23
+
+
+@pytest.mark.parametrize("where", [(0,), (1,), (0, 1), (0, 2), (1, 2)])
+@pytest.mark.parametrize("value", [float("inf"), float("nan"), 1e30])
+def test_plain_tiles_between_others(cuda, value, where):
+    """A CTA that takes several 128-row tiles, with values that send some of
+    them to the plain sums: those are the CUDA-core kernel's bits, the tiles
+    before and after them and their column sums stay what they are without."""
+    sms = torch.cuda.get_device_properties(cuda).multi_processor_count
+    M = 128 * (2 * sms + 5) + 77                 # three tiles on the first CTAs
+    g = torch.Generator().manual_seed(7)
+    A = torch.randn((M, 192), generator=g).to(cuda)
+    Bt = (torch.randn((192, 192), generator=g) / 14).to(cuda)
+    H = torch.randn((M, 192), generator=g).to(cuda)
+    clean, _ = _rowgemm(_rows(A, 192), Bt, H)
+    tiles = [w * sms + 3 for w in where]         # all on CTA 3
+    for t in tiles:
+        A[128 * t + 5, 17] = value
+        H[128 * t + 5] = 0                       # the row itself stays out of the column sums
+    split, sums = _rowgemm(_rows(A, 192), Bt, H)
+    plain, plain_sums = _rowgemm(_rows(A, 193), Bt, H)
+    special = torch.zeros(M, dtype=torch.bool, device=cuda)
+    for t in tiles:
+        special[128 * t:128 * (t + 1)] = True
+    assert torch.equal(_bits(split[special]), _bits(plain[special]))
+    assert torch.equal(_bits(split[~special]), _bits(clean[~special]))
+    # up to 2 * sms * 128 + rows of |c| <= 6: each side's additions round
+    assert bool(((sums.double().sum(0) - plain_sums.double().sum(0)).abs() <= 1e-6 * plain.abs().double().sum(0)).all())

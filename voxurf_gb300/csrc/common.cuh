@@ -279,13 +279,4 @@ __device__ __forceinline__ unsigned transmittance_step(bool keep, float alpha, A
   return live;
 }
 
-// First index i in [lo, hi) with a[i] >= key (a sorted ascending).
-__device__ __forceinline__ int64_t lower_bound_i64(const int64_t* a, int64_t lo, int64_t hi, int64_t key) {
-  while (lo < hi) {
-    int64_t mid = lo + ((hi - lo) >> 1);
-    if (a[mid] < key) lo = mid + 1; else hi = mid;
-  }
-  return lo;
-}
-
 }  // namespace vx

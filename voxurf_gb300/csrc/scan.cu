@@ -58,9 +58,8 @@ __global__ void __launch_bounds__(SCAN_THREADS) tile_reduce_kernel(const Tin* __
   }
 }
 
-// One CTA scans the tile sums in place (exclusive); writes the total.
-__global__ void __launch_bounds__(SCAN_THREADS) tile_sums_scan_kernel(int64_t* __restrict__ tile_sums, int64_t n_tiles,
-                                                                      int64_t* __restrict__ total_out) {
+// One CTA scans the tile sums in place (exclusive).
+__global__ void __launch_bounds__(SCAN_THREADS) tile_sums_scan_kernel(int64_t* __restrict__ tile_sums, int64_t n_tiles) {
   __shared__ int64_t warp_sums[SCAN_THREADS / 32];
   __shared__ int64_t chunk_total;
   int64_t carry = 0;
@@ -73,7 +72,6 @@ __global__ void __launch_bounds__(SCAN_THREADS) tile_sums_scan_kernel(int64_t* _
     carry += chunk_total;
     __syncthreads();
   }
-  if (threadIdx.x == 0) *total_out = carry;
 }
 
 template <typename Tin, typename Tout>
@@ -103,8 +101,9 @@ __global__ void __launch_bounds__(SCAN_THREADS) tile_scan_kernel(const Tin* __re
   if (blockIdx.x == gridDim.x - 1 && threadIdx.x == SCAN_THREADS - 1) out[n] = (Tout)ex;
 }
 
-// Up to SCAN_SMALL counts in one CTA: a chunk of SMALL_THREADS counts a step,
-// the next step's counts loaded ahead.
+// Up to SCAN_SMALL counts in one CTA, SMALL_THREADS x SMALL_ITEMS of them a step.
+// Three launches take about 16 us at any size up to there; one launch 6 us up to
+// 8,192 counts (one step) and 4 us more for every further step: 18 us at 32,768.
 constexpr int SMALL_THREADS = 1024;
 constexpr int SMALL_ITEMS = 8;
 constexpr int64_t SCAN_SMALL = 4 * SMALL_THREADS * SMALL_ITEMS;
@@ -142,6 +141,8 @@ __global__ void __launch_bounds__(SMALL_THREADS) scan_small_kernel(const Tin* __
 }
 
 int64_t scan_n_tiles(int64_t n) { return (n + SCAN_TILE - 1) / SCAN_TILE; }
+// (the scratch is one entry larger than the tile sums; callers size it by
+// vx_scan_scratch_bytes, which stays what it was)
 
 template <typename Tin, typename Tout>
 int exclusive_scan(const Tin* in, int64_t n, Tout* out, void* scratch, size_t scratch_bytes, cudaStream_t st) {
@@ -160,7 +161,7 @@ int exclusive_scan(const Tin* in, int64_t n, Tout* out, void* scratch, size_t sc
   }
   tile_reduce_kernel<Tin><<<(unsigned)nt, SCAN_THREADS, 0, st>>>(in, n, tiles);
   int s = launch_status(); if (s) return s;
-  tile_sums_scan_kernel<<<1, SCAN_THREADS, 0, st>>>(tiles, nt, tiles + nt);
+  tile_sums_scan_kernel<<<1, SCAN_THREADS, 0, st>>>(tiles, nt);
   s = launch_status(); if (s) return s;
   tile_scan_kernel<Tin, Tout><<<(unsigned)nt, SCAN_THREADS, 0, st>>>(in, n, tiles, out);
   return launch_status();
