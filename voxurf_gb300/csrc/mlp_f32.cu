@@ -343,9 +343,14 @@ struct SumJobs {
 // A block of 256 threads sums 32 V consecutive outputs of one row (a lane owns
 // V of them): warp w adds the partials of its contiguous eighth of k, then the
 // eight warp sums are added in warp order.  The order is fixed, so the result
-// does not depend on timing.  V = 4 where rows are whole float4s: a warp then
-// reads 512 bytes of a partial instead of 128, 147 KB apart.  rgbnet's five
-// sums: 42 us (with 2,047 mostly empty rows of column sums per layer) -> 17 us.
+// does not depend on timing.  V = 4 where rows are whole float4s and there are
+// SUM_VEC outputs or more: a warp then reads 512 bytes of a partial instead of
+// 128, 147 KB apart (rgbnet's five sums 42 us, with 2,047 mostly empty rows of
+// column sums per layer, -> 17 us).  The column sums of a layer are too few for
+// that: 64 outputs of 2,047 partials are one half-empty warp's work as float4s,
+// two full ones' as floats (18.5 against 12.3 us).
+constexpr int64_t SUM_VEC = 2048;
+
 template <int V>
 __device__ __forceinline__ void sum_outputs(const SumJob& S, float (&red)[8][32][4]) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -403,7 +408,7 @@ __device__ __forceinline__ void sum_outputs(const SumJob& S, float (&red)[8][32]
 __global__ void __launch_bounds__(256) sum_partials_kernel(SumJobs J) {
   const SumJob& S = J.j[blockIdx.y];
   __shared__ float red[8][32][4];
-  if (S.cols % 4 == 0 && S.part_ld % 4 == 0 && S.part_stride % 4 == 0 &&
+  if (S.rows * S.cols >= SUM_VEC && S.cols % 4 == 0 && S.part_ld % 4 == 0 && S.part_stride % 4 == 0 &&
       (reinterpret_cast<uintptr_t>(S.part) & 15) == 0)
     sum_outputs<4>(S, red);
   else
