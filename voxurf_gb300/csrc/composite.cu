@@ -54,14 +54,15 @@ __device__ __forceinline__ void ray_segment(const int64_t* __restrict__ ray_id, 
 }
 
 // 32-sample scans in flight per warp: as many as the segment fills, up to
-// four.  (Four for every segment: 1M rays of 1 to 5 samples 803 us forward and
-// 327 us backward with the even search above, where one scan and a bisection
-// took 667 and 278.)
+// four (one or two are a single step).  With four for every segment and the
+// even search above, 1M rays of 1 to 5 samples took 803 us forward and 327 us
+// backward, where one scan and a bisection took 656 and 287.
 template <typename F>
-__device__ __forceinline__ void by_chunks(int64_t len, F scan) {
-  if (len <= 32) scan(std::integral_constant<int, 1>());
-  else if (len <= 64) scan(std::integral_constant<int, 2>());
-  else scan(std::integral_constant<int, 4>());
+__device__ __forceinline__ void by_length(int64_t len, F scan) {
+  if (len <= 32) scan(0.f, std::integral_constant<int, 1>());
+  else if (len <= 64) scan(0.f, std::integral_constant<int, 2>());
+  else if (len <= VX_FP32_SCAN_MAX_STEPS) scan(0.f, std::integral_constant<int, 4>());
+  else scan(FloatPair(), std::integral_constant<int, 4>());
 }
 
 // Warp-level forward scan of one segment.  Writes weight/T for every sample
@@ -83,8 +84,10 @@ __device__ __forceinline__ void scan_segment_fwd(const float* __restrict__ alpha
     for (int c = 0; c < CHUNKS; ++c) {
       a[c] = nxt[c];
       incl[c] = Op::one_minus(a[c]);
-      const int64_t i = base + 32 * (CHUNKS + c) + lane;   // the next step's samples, while this one scans
-      nxt[c] = i < end ? alpha[i] : 0.f;
+      if (CHUNKS == 4) {                                   // the next step's samples, while this one scans
+        const int64_t i = base + 32 * (CHUNKS + c) + lane;
+        nxt[c] = i < end ? alpha[i] : 0.f;
+      }
     }
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1)
@@ -120,6 +123,7 @@ __device__ __forceinline__ void scan_segment_fwd(const float* __restrict__ alpha
         return;
       }
     }
+    if (CHUNKS < 4) break;   // the one step of a short segment
   }
   *i_end_out = end;
   *last_out = Op::value(carry);
@@ -143,10 +147,9 @@ __global__ void alpha2weight_kernel(const float* __restrict__ alpha, const int64
   }
   int64_t ie;
   float last;
-  if (end - beg > VX_FP32_SCAN_MAX_STEPS)
-    scan_segment_fwd<FloatPair, 4>(alpha, beg, end, weight, T, &ie, &last);
-  else
-    by_chunks(end - beg, [&](auto c) { scan_segment_fwd<float, c>(alpha, beg, end, weight, T, &ie, &last); });
+  by_length(end - beg, [&](auto acc, auto chunks) {
+    scan_segment_fwd<decltype(acc), chunks>(alpha, beg, end, weight, T, &ie, &last);
+  });
   if (lane_id() == 0) {
     i_start[r] = beg;
     i_end[r] = ie;
@@ -198,8 +201,9 @@ __device__ __forceinline__ void scan_segment_bwd(const float* __restrict__ alpha
       if (lane == 31) after = Op::of(0.f);
       const Acc back = carry + after;
       if (i >= beg) grad[i] = Op::grad(gw_t[c], back, a[c]);
-      carry = carry + warp_shfl(suffix[c], 0);
+      if (CHUNKS == 4 || c + 1 < CHUNKS) carry = carry + warp_shfl(suffix[c], 0);
     }
+    if (CHUNKS < 4) break;
   }
 }
 
@@ -219,12 +223,10 @@ __global__ void alpha2weight_backward_kernel(const float* __restrict__ alpha, co
     if (lane_id() == 0) set_device_error(err, VX_ERR_BOUNDS);
     return;
   }
-  if (end - beg > VX_FP32_SCAN_MAX_STEPS)
-    scan_segment_bwd<FloatPair, 4>(alpha, weight, T, grad_weights, beg, end, grad_last[r] * alphainv_last[r], grad);
-  else
-    by_chunks(end - beg, [&](auto c) {
-      scan_segment_bwd<float, c>(alpha, weight, T, grad_weights, beg, end, grad_last[r] * alphainv_last[r], grad);
-    });
+  const float back = grad_last[r] * alphainv_last[r];
+  by_length(end - beg, [&](auto acc, auto chunks) {
+    scan_segment_bwd<decltype(acc), chunks>(alpha, weight, T, grad_weights, beg, end, back, grad);
+  });
 }
 
 }  // namespace vx
