@@ -790,8 +790,10 @@ int vx_mlp_train_reduce(const vx_mlp_reduce_job* jobs, int n_jobs, void* stream)
 /* ---- colour-MLP training in plain FP32 (the same layers as above with FP32
  *      operands: fused multiply-adds on the CUDA cores, and for the backward
  *      GEMMs of widths 128 and 192 with aligned buffers the tensor cores on
- *      operands split into three BF16 parts, no less exact; the output layer
- *      runs in vx_mlp_head / vx_mlp_head_backward).  Weights enter as
+ *      operands split into three BF16 parts: rows and weight gradients as exact
+ *      as the CUDA-core sums, column sums of terms of one sign within a unit in
+ *      the last place; the output layer runs in vx_mlp_head /
+ *      vx_mlp_head_backward).  Weights enter as
  *      Bt [Kp][Np] FP32 (vx_mlp_train_pack mode 3), Np in {32, 64, 80, 128,
  *      192}. ---- */
 typedef struct {

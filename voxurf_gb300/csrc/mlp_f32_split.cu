@@ -1,5 +1,5 @@
 // The FP32 MLP backward on the tensor cores: FP32 operands as three BF16
-// parts each, FP32 accumulation kept as exact as the CUDA-core sums.
+// parts each, FP32 accumulation whose truncation is kept small.
 //
 // x = hi + mid + lo with hi = bf16(x), mid = bf16(x - hi), lo = bf16(x - hi -
 // mid): 3 x 8 significant bits, all 24 of an FP32 value.  The operands are
@@ -15,14 +15,14 @@
 //     products end the small sum; then the two are added in registers with
 //     rounding to nearest;
 //   * in the weight gradient a hi hi sum is 4 MMAs long, and every second one
-//     is truncated in the opposite direction (negated(), below).
+//     is truncated the other way (negated(), below).
 // Measured against 64 bits (test_f32_split_gpu.py, test_f32_split_range_gpu.py),
 // relative: rows x 192 x 192 9.3e-8 where the CUDA-core sums are at 2.5e-7, a
 // weight gradient over 131,003 rows 1.4e-7 against 3.7e-7.  On operands of one
 // sign, where truncation does not average out: rows 1.3e-7 against 2.1e-7, but
 // their column sums 1.2e-7 (one unit in the last place) against 2e-9; weight
 // gradients after their ordered sum 5.0e-8 both over 60,001 rows, 5.5e-8 against
-// 5.9e-8 over 131,003 (1.4e-7 with sums of 8 MMAs in one direction; 4 us less).
+// 5.9e-8 over 131,003 (1.4e-7 with sums of 8 MMAs in one direction; 2 us less).
 // The forward keeps its CUDA-core sums: a ReLU whose input lies within a
 // rounding of zero would switch with them.
 //
@@ -43,7 +43,7 @@
 //                         the others waiting, 105 -> 91 us), and the partials
 //                         leave in whole sectors (4 us).
 // 131,003 rows, 192 x 192: the row GEMM with mask and column sums 176 -> 84 us
-// (its three FP32 matrices take 44 us of HBM), the weight gradient 208 -> 91
+// (its three FP32 matrices take 44 us of HBM), the weight gradient 208 -> 92
 // us (30 us of HBM).  Bound now: the row GEMM's loads and stores beside its
 // MMAs; in the weight gradient the MMAs and the splitting of 32 rows, each
 // about 1 us, two stages deep, and about 10 us of filling and storing per CTA.
@@ -73,11 +73,11 @@ struct Split2 {
 __device__ __forceinline__ float bf16_lo(uint32_t p) { return __uint_as_float(p << 16); }
 __device__ __forceinline__ float bf16_hi(uint32_t p) { return __uint_as_float(p & 0xffff0000u); }
 
-__device__ __forceinline__ Split2 split2(float a, float b, bool& bad, float scale = SCALE) {
+__device__ __forceinline__ Split2 split2(float a, float b, bool& bad) {
   Split2 s;
   bad |= !(fabsf(a) < SPLIT_MAX) || !(fabsf(b) < SPLIT_MAX);
-  a *= scale;
-  b *= scale;
+  a *= SCALE;
+  b *= SCALE;
   s.hi = pack_bf16(a, b);
   a -= bf16_lo(s.hi);
   b -= bf16_hi(s.hi);
@@ -425,12 +425,13 @@ __device__ __forceinline__ void st_sector(float* p, const float* v) {
 constexpr int WS_ROWS = 32;         // rows per stage
 constexpr int WS_SLOTS = 2;         // stages of split operands
 constexpr int WS_RAW = 3;           // stages of FP32 rows on their way
-constexpr int WS_GROUP = 2;         // stages summed before the registers take them: hi hi sums of 4 MMAs
+constexpr int WS_GROUP = 2;         // stages between two reads of the hi hi sums: 4 MMAs
+constexpr int WS_SMALL = 8;         // and of the small ones
 
 // An MMA truncates its running sum, which for products of one sign always falls
-// short.  So every other group is subtracted from the sum of the one before it
-// (its A is negated): that sum D1 shrinks to D2 = D1 - S2 and is truncated the
-// other way, and the two groups together are 2 D1 - D2.
+// short.  So every other group of hi hi products is subtracted from the sum of
+// the one before it (the MMA negates A): that sum D1 shrinks to D2 = D1 - S2 and
+// is truncated the other way, and the two groups together are 2 D1 - D2.
 __device__ __forceinline__ bool negated(int st) { return (st / WS_GROUP) & 1; }
 
 // M columns of A, NC of B: MN-major tiles of 8 x 8 values, 8 rows of K a block
@@ -523,8 +524,8 @@ __global__ void __launch_bounds__(WgradGeo<M, NC>::THREADS + 32, 1) split_wgrad_
       cp_async16(dst + (G::A_ITEMS + q) * G::THREADS, n ? b_src[q] + row * P.ldb : P.A, (uint32_t)(4 * n));
     }
   };
-  auto put = [&](uint8_t* dst, int step, const float4& x, bool& bad, float scale) {
-    const Split2 s0 = split2(x.x, x.y, bad, scale), s1 = split2(x.z, x.w, bad, scale);
+  auto put = [&](uint8_t* dst, int step, const float4& x, bool& bad) {
+    const Split2 s0 = split2(x.x, x.y, bad), s1 = split2(x.z, x.w, bad);
     *reinterpret_cast<uint2*>(dst) = make_uint2(s0.hi, s1.hi);
     *reinterpret_cast<uint2*>(dst + step) = make_uint2(s0.mid, s1.mid);
     *reinterpret_cast<uint2*>(dst + 2 * step) = make_uint2(s0.lo, s1.lo);
@@ -538,13 +539,7 @@ __global__ void __launch_bounds__(WgradGeo<M, NC>::THREADS + 32, 1) split_wgrad_
 #pragma unroll
       for (int e = 0; e < 16; ++e) acc[mt][b][e] = 0.f;
   bool ok = true, bad = false;
-  // adds the group that ends with stage st to the registers
-  auto drain = [&](int st) {
-    const bool paired = (st / WS_GROUP + 1) * WS_GROUP < nst;       // another group follows
-    const float unit = negated(st) ? -UNSCALE : (paired ? 2.f * UNSCALE : UNSCALE);
-    ok = mbar_wait(bar + st % WS_SLOTS, (uint32_t)((st / WS_SLOTS) & 1)) && ok;
-    fence_after();
-    __syncwarp();
+  auto add = [&](uint32_t col, float unit) {
 #pragma unroll
     for (int mt = 0; mt < G::MT; ++mt) {
       if (mt * TILE_M + 32 * quarter >= M) break;   // warp-uniform: lanes past the last column of A
@@ -552,14 +547,21 @@ __global__ void __launch_bounds__(WgradGeo<M, NC>::THREADS + 32, 1) split_wgrad_
       for (int b = 0; b < G::BLOCKS; ++b) {
         const int c = 16 * (G::PARTS * b + part);
         if (c >= NC) break;
-        uint32_t s[16], h[16];
-        ld_cols<16>(tm_lanes + (uint32_t)(mt * NC + c), s);
-        ld_cols<16>(tm_lanes + (uint32_t)(G::D_HI + mt * NC + c), h);
+        uint32_t s[16];
+        ld_cols<16>(tm_lanes + col + (uint32_t)(mt * NC + c), s);
 #pragma unroll
-        for (int e = 0; e < 16; ++e)
-          acc[mt][b][e] = fmaf(unit, __uint_as_float(s[e]) + __uint_as_float(h[e]), acc[mt][b][e]);
+        for (int e = 0; e < 16; ++e) acc[mt][b][e] = fmaf(unit, __uint_as_float(s[e]), acc[mt][b][e]);
       }
     }
+  };
+  // adds the groups that end with stage st to the registers
+  auto drain = [&](int st) {
+    const bool paired = (st / WS_GROUP + 1) * WS_GROUP < nst;       // another group follows
+    ok = mbar_wait(bar + st % WS_SLOTS, (uint32_t)((st / WS_SLOTS) & 1)) && ok;
+    fence_after();
+    __syncwarp();
+    if ((st + 1) % WS_SMALL == 0 || st == nst - 1) add(0, UNSCALE);
+    add(G::D_HI, negated(st) ? -UNSCALE : (paired ? 2.f * UNSCALE : UNSCALE));
   };
 
   if (warp < G::WARPS) {
@@ -572,15 +574,14 @@ __global__ void __launch_bounds__(WgradGeo<M, NC>::THREADS + 32, 1) split_wgrad_
       const int slot = st % WS_SLOTS;
       if (st >= WS_SLOTS) ok = mbar_wait(bar + slot, (uint32_t)((st / WS_SLOTS - 1) & 1)) && ok;
       asm volatile("cp.async.wait_group %0;" ::"n"(WS_RAW - 1) : "memory");
-      const float scale = negated(st) ? -SCALE : SCALE;
       uint8_t* base = smem + (size_t)slot * G::SLOT;
       const float4* mine = raw + (size_t)(st % WS_RAW) * (G::ITEMS * G::THREADS) + tid;
 #pragma unroll
-      for (int q = 0; q < G::A_ITEMS; ++q) put(base + a_dst + q * (M * 16), G::A_PART, mine[q * G::THREADS], bad, scale);
+      for (int q = 0; q < G::A_ITEMS; ++q) put(base + a_dst + q * (M * 16), G::A_PART, mine[q * G::THREADS], bad);
 #pragma unroll
       for (int q = 0; q < G::B_ITEMS; ++q)
         if (b_row[q] >= 0)
-          put(base + 3 * G::A_PART + b_dst[q], G::B_PART, mine[(G::A_ITEMS + q) * G::THREADS], bad, SCALE);
+          put(base + 3 * G::A_PART + b_dst[q], G::B_PART, mine[(G::A_ITEMS + q) * G::THREADS], bad);
       if (st + WS_RAW < nst) load(st + WS_RAW);
       cp_async_commit();
       if (st > 0 && st % WS_GROUP == 0) drain(st - 1);
@@ -602,7 +603,8 @@ __global__ void __launch_bounds__(WgradGeo<M, NC>::THREADS + 32, 1) split_wgrad_
         const uint32_t a_s = smem_u32(smem + (size_t)slot * G::SLOT);
         // (a descriptor's address field holds 16-byte units and does not carry)
         const uint64_t a_d = desc(a_s, M * 16, 128), b_d = desc(a_s + 3 * G::A_PART, NC * 16, 128);
-        const bool first = st % (2 * WS_GROUP) == 0;
+        const uint32_t id_hh = negated(st) ? id | IDESC_NEGATE_A : id;
+        const bool first_hh = st % (2 * WS_GROUP) == 0, first_small = st % WS_SMALL == 0;
 #pragma unroll
         for (int mt = 0; mt < G::MT; ++mt)
 #pragma unroll
@@ -612,8 +614,8 @@ __global__ void __launch_bounds__(WgradGeo<M, NC>::THREADS + 32, 1) split_wgrad_
 #pragma unroll
             for (int ks = 0; ks < WS_ROWS / 16; ++ks)
               mma_ss(d, a_d + (uint64_t)((pa[q] * G::A_PART + 2 * ks * (M * 16) + mt * 16 * 128) / 16),
-                     b_d + (uint64_t)((pb[q] * G::B_PART + 2 * ks * (NC * 16)) / 16), id,
-                     !first || ks > 0 || (!hh && q > 0));
+                     b_d + (uint64_t)((pb[q] * G::B_PART + 2 * ks * (NC * 16)) / 16), hh ? id_hh : id,
+                     ks > 0 || (hh ? !first_hh : !first_small || q > 0));
           }
         commit(bar + slot);
       }

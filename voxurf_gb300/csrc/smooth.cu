@@ -272,8 +272,8 @@ __global__ void __launch_bounds__(SM_THREADS, 3) smooth_march_kernel(const float
 // the same products in the same order as the kernel above: the bits are equal.
 // Bound: L2 reads (each row is read by two warps) and their latency; 74 thread
 // instructions an output became about 20.  The planes arrive by cp.async, three
-// deep.  Five taps, inputs from HBM: 256^3 forward 55 -> 36 us, adjoint 77 -> 50 us
-// (20 us of HBM); 384^3 149 -> 101 and 221 -> 138 us.
+// deep.  Five taps, inputs from HBM: 256^3 forward 55 -> 35 us, adjoint 77 -> 50 us
+// (20 us of HBM); 384^3 149 -> 100 and 221 -> 137 us.
 constexpr int SR_WARPS = 4;      // consecutive y tiles share rows through L1
 constexpr int SR_Z = 128;
 constexpr int SR_STAGES = 3;     // planes on their way or in use

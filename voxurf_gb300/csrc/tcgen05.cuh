@@ -41,6 +41,8 @@ __host__ __device__ constexpr uint32_t idesc(int M, int N, int a_mn = 0, int b_m
          ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
+constexpr uint32_t IDESC_NEGATE_A = 1u << 13;   // D (+)= -A B
+
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
 }

@@ -8,9 +8,9 @@ Two native engines, both hand-written sm_103a kernels:
   kernels of mlp_train.cu (BF16 operands, FP32 accumulation);
 * FP32 rows (the plain path): F32TrainMLP, FP32 CUDA-core kernels
   (mlp_f32.cu) for the hidden layers' forward, their backward on the tensor
-  cores with every FP32 operand in three BF16 parts (mlp_f32_split.cu, no less
-  exact than the CUDA-core sums), and the fused output-layer kernels of
-  mlp_ops.cu (vx_mlp_head, vx_mlp_head_backward).
+  cores with every FP32 operand in three BF16 parts (mlp_f32_split.cu, whose
+  header has its errors beside the CUDA-core sums'), and the fused output-layer
+  kernels of mlp_ops.cu (vx_mlp_head, vx_mlp_head_backward).
 Parameters stay FP32 masters (the reference's nn.Linear parameters, same
 names and shapes); each forward refreshes the engine's operand copies of
 them with one pack launch, and the backward returns FP32 gradients.
