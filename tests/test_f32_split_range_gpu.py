@@ -130,3 +130,21 @@ def test_plain_tiles_between_others(cuda, value, where):
     assert torch.equal(_bits(split[~special]), _bits(clean[~special]))
     # up to 2 * sms * 128 + rows of |c| <= 6: each side's additions round
     assert bool(((sums.double().sum(0) - plain_sums.double().sum(0)).abs() <= 1e-6 * plain.abs().double().sum(0)).all())
+
+
+def test_plain_tiles_do_not_depend_on_timing(cuda):
+    """Large finite values: the column sums of a tile that is summed plainly
+    are added in one order, its even rows, then its odd rows."""
+    g = torch.Generator().manual_seed(8)
+    A = torch.randn((39 * 128, 192), generator=g).to(cuda)
+    A[::100, 3] = 1e12                           # one in every tile
+    Bt = torch.randn((192, 192), generator=g).to(cuda)
+    H = torch.randn(A.shape, generator=g).to(cuda)
+    split, sums = _rowgemm(_rows(A, 192), Bt, H)
+    plain, _ = _rowgemm(_rows(A, 193), Bt, H)
+    assert torch.equal(_bits(split), _bits(plain))
+    c = split.view(39, 64, 2, 192)
+    want = torch.zeros((39, 2, 192), device=cuda)
+    for r in range(64):
+        want += c[:, r]
+    assert torch.equal(sums[:39], want[:, 0] + want[:, 1])

@@ -130,21 +130,31 @@ __device__ __forceinline__ void load_chunk(const RowGemmParams& P, int64_t row0,
   }
 }
 
-// A tile by plain FP32 sums, as the CUDA-core kernel forms them.
+// A tile by plain FP32 sums, as the CUDA-core kernel forms them.  The column
+// sums are added in an order of their own too: a thread's rows, then the groups
+// of threads (red: [4][N], free until the last tile).
 template <int K, int N>
-__device__ __noinline__ void plain_tile(const RowGemmParams& P, int64_t m0, int64_t M, float* extra) {
-  for (int i = threadIdx.x; i < TILE_M * N; i += SP_THREADS) {
-    const int64_t row = m0 + i / N;
-    const int col = i % N;
-    if (row >= M) return;
-    float v = 0.f;
-    for (int k = 0; k < K; ++k) v = fmaf(P.A[row * P.lda + k], P.Bt[(int64_t)k * N + col], v);
-    if (P.mode == 1) {
-      v = P.H[row * P.ldh + col] > 0.f ? v : 0.f;
-      atomicAdd(extra + col, v);
+__device__ __noinline__ void plain_tile(const RowGemmParams& P, int64_t m0, int64_t M, float* extra, float* red) {
+  constexpr int GROUPS = SP_THREADS / N < 4 ? SP_THREADS / N : 4;
+  const int col = threadIdx.x % N, group = threadIdx.x / N;
+  if (group < GROUPS) {
+    const int64_t end = min(M, m0 + TILE_M);
+    float sum = 0.f;
+    for (int64_t row = m0 + group; row < end; row += GROUPS) {
+      float v = 0.f;
+      for (int k = 0; k < K; ++k) v = fmaf(P.A[row * P.lda + k], P.Bt[(int64_t)k * N + col], v);
+      if (P.mode == 1) {
+        v = P.H[row * P.ldh + col] > 0.f ? v : 0.f;
+        sum += v;
+      }
+      if (col < P.n_store) P.C[row * P.ldc + col] = v;
     }
-    if (col < P.n_store) P.C[row * P.ldc + col] = v;
+    red[group * N + col] = sum;
   }
+  __syncthreads();
+  for (int n = threadIdx.x; n < N; n += SP_THREADS)
+    for (int g = 0; g < GROUPS; ++g) extra[n] += red[g * N + n];
+  __syncthreads();
 }
 
 template <int K, int N>
@@ -306,7 +316,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1) split_rowgemm_kernel(RowGemmPar
     fence_after();
     if (P.mode == 1) take_h(G::CHUNKS - 1);
     if (plain) {
-      plain_tile<K, N>(P, tile * TILE_M, M, extra);
+      plain_tile<K, N>(P, tile * TILE_M, M, extra, red);
       continue;
     }
     // ---- the tile's outputs: both sums, mask, store ----
