@@ -4,7 +4,7 @@ import pytest
 import torch
 
 from test_f32_split_gpu import _err, _rowgemm, _rows, _wgrad
-from voxurf_gb300 import _abi
+from voxurf_gb300 import _abi, _native
 from voxurf_gb300._torch import ptr, stream_ptr
 
 pytestmark = pytest.mark.gpu
@@ -148,3 +148,26 @@ def test_plain_tiles_do_not_depend_on_timing(cuda):
     for r in range(64):
         want += c[:, r]
     assert torch.equal(sums[:39], want[:, 0] + want[:, 1])
+
+
+@pytest.mark.parametrize("special", [False, True])
+@pytest.mark.parametrize("mode", [1, 2])
+def test_rowgemm_in_place(cuda, mode, special):
+    """C over A, as the CUDA-core kernel allows: every row from its own values
+    before the call."""
+    sms = torch.cuda.get_device_properties(cuda).multi_processor_count
+    M = 128 * (sms + 3)
+    g = torch.Generator().manual_seed(9)
+    A = torch.randint(-3, 4, (M, 192), generator=g).float().to(cuda)
+    Bt = torch.randint(-3, 4, (192, 192), generator=g).float().to(cuda)
+    H = torch.randint(-1, 2, (M, 192), generator=g).float().to(cuda)
+    if special:
+        A[::200, 9] = float("inf")
+        Bt[9] = Bt[9].abs() + 1                  # infinite rows, no NaN
+    want, _ = _rowgemm(_rows(A, 193), Bt, H if mode == 1 else None)
+    colsum = torch.empty((int(_native.load().vx_mlp_f32_rowgemm_grid(M)), 192), device=cuda)
+    a = _abi.MlpF32RowGemmArgs()
+    a.M, a.K, a.A, a.lda, a.Bt, a.Np, a.mode = M, 192, ptr(A), 192, ptr(Bt), 192, mode
+    a.H, a.ldh, a.C, a.ldc, a.n_store, a.colsum, a.colsum_cap = ptr(H), 192, ptr(A), 192, 192, ptr(colsum), colsum.numel()
+    _abi.call_struct("vx_mlp_f32_rowgemm", a, stream_ptr(cuda))
+    assert torch.equal(_bits(A), _bits(want))

@@ -392,11 +392,21 @@ __global__ void __launch_bounds__(SP_THREADS, 1) split_rowgemm_kernel(RowGemmPar
   }
 }
 
+// Whether C's rows share memory with A's.  A CTA here reads the first columns of
+// its next tile while it writes this one, through the read-only path, and forms
+// plain tiles element by element from A; the CUDA-core kernel has read all of a
+// tile's A when it writes it, and takes such calls.
+static bool in_place(const RowGemmParams& P) {
+  const float *a1 = P.A + (P.M - 1) * P.lda + P.K, *c1 = P.C + (P.M - 1) * P.ldc + P.n_store;
+  return P.M > 0 && P.A < c1 && P.C < a1;
+}
+
 bool split_rowgemm_takes(const RowGemmParams& P) {
   const uintptr_t a16 = reinterpret_cast<uintptr_t>(P.A), c8 = reinterpret_cast<uintptr_t>(P.C) |
                                                                reinterpret_cast<uintptr_t>(P.mode == 1 ? P.H : nullptr);
   return P.mode != 0 && (P.K == 128 || P.K == 192) && (P.Np == P.K || P.Np == 80 || P.Np == 64) && P.lda % 4 == 0 &&
-         a16 % 16 == 0 && c8 % 8 == 0 && P.ldc % 2 == 0 && (P.mode != 1 || (P.ldh % 2 == 0 && P.n_store == P.Np));
+         a16 % 16 == 0 && c8 % 8 == 0 && P.ldc % 2 == 0 && (P.mode != 1 || (P.ldh % 2 == 0 && P.n_store == P.Np)) &&
+         !in_place(P);
 }
 
 unsigned split_rowgemm_grid(int64_t M) {
