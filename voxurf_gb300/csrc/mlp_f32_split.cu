@@ -397,8 +397,9 @@ __global__ void __launch_bounds__(SP_THREADS, 1) split_rowgemm_kernel(RowGemmPar
 // plain tiles element by element from A; the CUDA-core kernel has read all of a
 // tile's A when it writes it, and takes such calls.
 static bool in_place(const RowGemmParams& P) {
+  if (P.M <= 0) return false;
   const float *a1 = P.A + (P.M - 1) * P.lda + P.K, *c1 = P.C + (P.M - 1) * P.ldc + P.n_store;
-  return P.M > 0 && P.A < c1 && P.C < a1;
+  return P.A < c1 && P.C < a1;
 }
 
 bool split_rowgemm_takes(const RowGemmParams& P) {
